@@ -1111,6 +1111,15 @@ int pasc_gb300_polish(pasc_gb300_problem *p, const pasc_gb300_polish_opts *o, pa
     };
     double f = 0.0;
     ACHK(objective(&f));
+    // the FP32 state's rows sum to 1 within rounding only, which moves f by up to 1e-8 relative,
+    // and a round that projects some of them back onto the simplex moves it again: the rounds
+    // start, and f is compared, on rows that sum to 1.  (A non-finite gamma is left as it is: the
+    // first round reports it.)
+    if (mixed && o->rounds > 0 && isfinite(f)) {
+        ACU(launch_project_f64(gam, p->T, p->K, s));
+        launches++;
+        ACHK(objective(&f));
+    }
     for (int r = 0; r < o->rounds; r++) {
         memset(h, 0, sizeof *h);
         h->tol = o->cg_tol;
