@@ -217,14 +217,15 @@ int pasc_gb300_spgqp_last_iterate(pasc_gb300_problem *p, double *ms, int *launch
 
 /* Sweep kernel of the mixed path (no reference counterpart: the reference has one SpMV and
  * separate vector kernels).  0 = one timestep per thread; 1 = tiles of 4 timesteps per
- * thread brought in by bulk asynchronous copies; -1 (default) = whichever is faster on the
- * first solve, measured on the solve's own first sweep. */
+ * thread brought in by bulk asynchronous copies; -1 (default) = where the signal's state fits in
+ * the GPU's shared memory, whole solves in one cooperative launch (reported as kernel 1), else
+ * whichever of the two is faster on the first solve, measured on the solve's own first sweep. */
 int pasc_gb300_set_sweep_variant(pasc_gb300_problem *p, int variant);
 int pasc_gb300_get_sweep_variant(pasc_gb300_problem *p, int *variant);
 /* The sweep configuration in use: kernel (-1 before the first solve), blocks of its grid,
  * and the sweep time (ms) the tuner measured for it (0 when pinned or taken from an earlier
- * problem of the same shape).  With variant -1 the first solve times both kernels at every
- * grid of 1, 2, ... blocks per SM up to their occupancy, on the solve's own start point
+ * problem of the same shape, or for a solve in one cooperative launch).  With variant -1 the
+ * first solve of a larger signal times both kernels at every grid of 1, 2, ... blocks per SM up to their occupancy, on the solve's own start point
  * (gamma is saved and restored around the timing runs). */
 int pasc_gb300_get_sweep_tuning(pasc_gb300_problem *p, int *variant, int *blocks, double *sweep_ms);
 

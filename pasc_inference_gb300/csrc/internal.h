@@ -64,6 +64,28 @@ struct SweepArgs {
     int swz = 0, roff = 0;
 };
 
+// A whole SPG solve in one cooperative launch, state in shared memory (kernels_resident.cu).
+struct ResidentPlan {
+    int blocks, threads;
+    int C, M;     // timesteps per block (the last one has the rest) and per thread
+    size_t smem;  // dynamic shared memory
+};
+
+struct ResidentArgs {
+    float *x;           // gamma, in place
+    const float *data;  // T (modes 0, 2)
+    const float *bmat;  // T*K (mode 1)
+    const float *theta, *kw;
+    SpgDevState *st;
+    unsigned long long *slots;  // resident_words(sms) words
+    unsigned int tag;           // of the launch's first sweep; a word of an earlier launch never carries it
+    long T;
+    int C, M;
+    long edge_lo, edge_hi;  // timesteps of the bulk-copy sweep's tiles without range checks
+    int init;    // the first sweep is the INIT sweep (project x, objective, first direction)
+    int sweeps;  // at most this many (the solve may end earlier)
+};
+
 // Graph (R > 1) mode, mixed path (graph.cu): x and d ping-pong, buffer st->cur current.
 struct GraphSweepArgs {
     const float *data;        // T*R
@@ -217,6 +239,12 @@ cudaError_t sweep_tma_make_rowmap(CUtensorMap *map, const float *base, long n, i
 int sweep_tma_threads(int K);
 bool sweep_tma_rows16(int K);
 cudaError_t launch_sweep_tma(int K, bool init, int grid, const SweepArgs &a, cudaStream_t s);
+// Resident solve: mode 0 data, 1 materialised b, 2 theta in the penalty.  False: the state does
+// not fit in the shared memory of `sms` SMs.
+bool resident_plan(int K, int mode, long T, int sms, int smem_optin, ResidentPlan *plan);
+cudaError_t resident_prepare(int K, int mode, const ResidentPlan &plan);  // attributes, co-residency check
+cudaError_t launch_resident(int K, int mode, const ResidentPlan &plan, const ResidentArgs &a, cudaStream_t s);
+size_t resident_words(int sms);
 cudaError_t launch_theta_f32(int K, int grid, const ThetaArgs &a, cudaStream_t s);
 cudaError_t launch_project_f32(float *x, long T, int K, cudaStream_t s);
 cudaError_t launch_matmult_f32(const float *x, float *y, long T, int K, float coeff, cudaStream_t s);

@@ -68,7 +68,7 @@ static void free_all(pasc_gb300_problem *p)
                    p->d, p->Ad, p->b, p->data32_raw, p->theta32, p->xb_raw[0], p->xb_raw[1], p->st,
                    p->partials, p->xbf, p->xnorm, p->bmat_raw, p->theta_split, p->theta_f32, p->tnorm,
                    p->mc_partials, p->mc_err, p->tp_ck64, p->tp_kw32, p->gptr, p->gidx, p->db_raw[0],
-                   p->db_raw[1], p->gpartials, p->stage32};
+                   p->db_raw[1], p->gpartials, p->stage32, p->res_slots};
     for (void *q : dev)
         if (q) cudaFree(q);
     if (p->st_h) cudaFreeHost(p->st_h);
@@ -195,6 +195,7 @@ int pasc_gb300_create(pasc_gb300_problem **out, long T, int K, int xdim, int pre
     auto bail = [&](int code) { free_all(p); return code; };
     if (cudaSetDevice(device) != cudaSuccess) return bail(fail(PASC_ERR_CUDA, "cudaSetDevice failed"));
     cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, device);
+    cudaDeviceGetAttribute(&p->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&p->ev0) != cudaSuccess || cudaEventCreate(&p->ev1) != cudaSuccess)
         return bail(fail(PASC_ERR_CUDA, "create: stream/event creation failed"));
@@ -1110,13 +1111,104 @@ static int autotune_variant(pasc_gb300_problem *p)
     return PASC_OK;
 }
 
-// spgqpsolver.cpp:104-137 plus the first direction (one INIT sweep)
-static int mixed_start(pasc_gb300_problem *p)
+// Whether the solve about to start runs as one cooperative launch with its state in shared memory
+// (kernels_resident.cu): the kernel is left to the library, and the state fits.
+static int resident_choose(pasc_gb300_problem *p)
+{
+    p->res_used = false;
+    if (p->graph || p->variant >= 0 || p->res_refused) return PASC_OK;
+    const int mode = p->bmat ? 1 : (p->tp ? 2 : 0);
+    if (p->res_mode != mode) {
+        p->res_mode = mode;
+        p->res_fits = resident_plan(p->K, mode, p->T, p->sms, p->smem_optin, &p->res_plan) &&
+                      resident_prepare(p->K, mode, p->res_plan) == cudaSuccess;
+        if (!p->res_fits) cudaGetLastError();
+    }
+    if (!p->res_fits) return PASC_OK;
+    if (!p->res_slots) {
+        const size_t n = resident_words(p->sms);
+        CHK(dalloc(&p->res_slots, n));
+        CU(cudaMemsetAsync(p->res_slots, 0, n * sizeof *p->res_slots, p->stream));
+    }
+    p->res_used = true;
+    return PASC_OK;
+}
+
+// sweeps of one launch at most: other work on the GPU gets its turn between launches
+static constexpr int RESIDENT_MAX_SWEEPS = 4096;
+
+// n sweeps (with init the INIT sweep first) while the solve runs.  res_used is cleared, and
+// nothing done, if the device refuses the cooperative launch (an SM partition, say).
+static int resident_run(pasc_gb300_problem *p, bool init, long n)
+{
+    cudaStream_t s = p->stream;
+    SpgDevState *h = p->st_h;
+    long left = n + (init ? 1 : 0);
+    int launches = 0;
+    if (init) {
+        fill_device_state(p, h);
+        CU(cudaMemcpyAsync(p->st, h, sizeof(SpgDevState), cudaMemcpyHostToDevice, s));
+    }
+    CU(cudaEventRecord(p->ev0, s));
+    do {
+        ResidentArgs a;
+        a.x = p->xb[p->cur];
+        a.data = p->data32;
+        a.bmat = p->bmat;
+        a.theta = p->theta32;
+        a.kw = p->tp ? p->tp_kw32 : nullptr;
+        a.st = p->st;
+        a.slots = p->res_slots;
+        a.T = p->T;
+        a.C = p->res_plan.C;
+        a.M = p->res_plan.M;
+        // tile k covers W owned timesteps from k*W on; with its halo of 4 on both sides it needs no
+        // range check if it starts after 0 and ends before T - 1
+        const long W = sweep_tma_tile_width(), k_edge = p->T > W + 5 ? (p->T - W - 5) / W + 1 : 0;
+        a.edge_lo = W;
+        a.edge_hi = k_edge * W;
+        a.init = init && launches == 0 ? 1 : 0;
+        a.sweeps = (int)(left < RESIDENT_MAX_SWEEPS ? left : RESIDENT_MAX_SWEEPS);
+        a.tag = p->res_tag;
+        cudaError_t e = launch_resident(p->K, p->res_mode, p->res_plan, a, s);
+        if (e == cudaErrorCooperativeLaunchTooLarge && launches == 0) {
+            cudaGetLastError();
+            p->res_refused = true;
+            p->res_used = false;
+            return PASC_OK;
+        }
+        if (e != cudaSuccess) return fail(PASC_ERR_CUDA, "resident solve: %s", cudaGetErrorString(e));
+        p->res_tag += (unsigned int)a.sweeps;
+        left -= a.sweeps;
+        launches++;
+        CU(cudaEventRecord(p->ev1, s));
+        CU(cudaMemcpyAsync(h, p->st, sizeof(SpgDevState), cudaMemcpyDeviceToHost, s));
+        CU(cudaStreamSynchronize(s));
+    } while (left > 0 && h->status == PASC_SPG_RUNNING && !h->error);
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, p->ev0, p->ev1);
+    p->run.launches += launches;
+    p->run.time_s += ms * 1e-3;
+    if (!init) {
+        p->run.last_iterate_ms = ms;
+        p->run.last_iterate_launches = launches;
+    }
+    CHK(check_device_error(p));
+    sync_run_from_device(p);
+    return PASC_OK;
+}
+
+// spgqpsolver.cpp:104-137 plus the first direction (one INIT sweep); a resident solve makes its
+// first `sweeps` iterations in the same launch
+static int mixed_start(pasc_gb300_problem *p, long sweeps)
 {
     const pasc_gb300_spgqp_opts *o = &p->run.o;
     if (o->stop_normgp_normb || o->stop_Anormgp_normb)
         return fail(PASC_ERR_NOTSUPP, "spgqp: ||b||-scaled stopping tests need the fp64 path");
     cudaStream_t s = p->stream;
+    CHK(resident_choose(p));
+    if (p->res_used) CHK(resident_run(p, true, sweeps));
+    if (p->res_used) return PASC_OK;
     CHK(autotune_variant(p));
     CHK(ensure_chunk_graph(p));
     SpgDevState *h = p->st_h;
@@ -1148,9 +1240,15 @@ static int mixed_iterate(pasc_gb300_problem *p, long n, int poll)
     sweep_args(p, &a);
     SpgDevState *h = p->st_h;
     if (p->run.status != PASC_SPG_RUNNING) return PASC_OK;
-    CHK(ensure_chunk_graph(p));
     const long room = p->run.o.maxit - p->run.it;
     if (n > room) n = room;
+    if (p->res_used) {
+        if (n > 0) CHK(resident_run(p, false, n));
+        if (!p->res_used) return fail(PASC_ERR_STATE, "spgqp_iterate: the device no longer takes the cooperative launch this solve began with");
+        if (p->run.status == PASC_SPG_RUNNING && p->run.it >= p->run.o.maxit) p->run.status = PASC_SPG_MAXIT;
+        return PASC_OK;
+    }
+    CHK(ensure_chunk_graph(p));
     long done = 0;
     int step = 0;
     const int sched[] = {2, 4, 8};
@@ -1194,12 +1292,13 @@ static int check_opts(const pasc_gb300_spgqp_opts *o)
     return PASC_OK;
 }
 
-static int spgqp_start(pasc_gb300_problem *p, const pasc_gb300_spgqp_opts *o)
+// sweeps: iterations that will follow at once (a resident solve makes them in its first launch)
+static int spgqp_start(pasc_gb300_problem *p, const pasc_gb300_spgqp_opts *o, long sweeps)
 {
     p->run = SpgRun();
     p->run.o = *o;
     p->run.started = true;
-    return p->precision == PASC_PREC_FP64 ? fp64_start(p) : mixed_start(p);
+    return p->precision == PASC_PREC_FP64 ? fp64_start(p) : mixed_start(p, sweeps);
 }
 
 static int spgqp_iterate(pasc_gb300_problem *p, long n, int poll)
@@ -1213,7 +1312,7 @@ int pasc_gb300_spgqp_start(pasc_gb300_problem *p, const pasc_gb300_spgqp_opts *o
     if (p->fem_inner) return fail(PASC_ERR_NOTSUPP, "spgqp_start: a reduced (fem_reduce < 1) problem solves with spgqp_solve");
     CHK(check_opts(o));
     CU(cudaSetDevice(p->device));
-    return spgqp_start(p, o);
+    return spgqp_start(p, o, 0);
 }
 
 int pasc_gb300_spgqp_iterate(pasc_gb300_problem *p, long n, int poll, pasc_gb300_spgqp_stats *st)
@@ -1259,7 +1358,7 @@ int pasc_gb300_spgqp_solve(pasc_gb300_problem *p, const pasc_gb300_spgqp_opts *o
         if (st) *st = ist;
         return PASC_OK;
     }
-    CHK(spgqp_start(p, o));
+    CHK(spgqp_start(p, o, o->maxit));
     CHK(spgqp_iterate(p, o->maxit, 1));
     if (p->run.status == PASC_SPG_RUNNING) p->run.status = PASC_SPG_MAXIT;
     fill_stats(p->run, st);
@@ -1431,6 +1530,7 @@ int pasc_gb300_set_sweep_variant(pasc_gb300_problem *p, int variant)
     if (variant == 1 && p->graph && p->img_W == 0)
         return fail(PASC_ERR_NOTSUPP, "set_sweep_variant: the fused image sweep needs T = 1 on a pixel grid (H >= 2)");
     p->variant = variant;
+    p->res_used = false;
     p->run.started = false;
     // a pinned kernel runs at full occupancy; -1 tunes kernel and grid again
     for (int v = 0; v < 2; v++) {
@@ -1444,9 +1544,9 @@ int pasc_gb300_set_sweep_variant(pasc_gb300_problem *p, int variant)
 int pasc_gb300_get_sweep_tuning(pasc_gb300_problem *p, int *variant, int *blocks, double *sweep_ms)
 {
     if (!p || !variant || !blocks || !sweep_ms) return fail(PASC_ERR_ARG, "get_sweep_tuning: NULL argument");
-    *variant = p->variant;
+    *variant = p->variant < 0 && p->res_used ? 1 : p->variant;
     const int v = p->variant < 0 ? 1 : p->variant;
-    *blocks = p->tp ? p->grid_sweep_tp[v] : p->grid_sweep[v];
+    *blocks = p->res_used ? p->res_plan.blocks : (p->tp ? p->grid_sweep_tp[v] : p->grid_sweep[v]);
     *sweep_ms = p->tune_ms;
     return PASC_OK;
 }
@@ -1576,7 +1676,7 @@ int pasc_gb300_get_residual_engine(pasc_gb300_problem *p, int *engine)
 int pasc_gb300_get_sweep_variant(pasc_gb300_problem *p, int *variant)
 {
     if (!p || !variant) return fail(PASC_ERR_ARG, "get_sweep_variant: NULL argument");
-    *variant = p->variant;
+    *variant = p->variant < 0 && p->res_used ? 1 : p->variant;
     return PASC_OK;
 }
 

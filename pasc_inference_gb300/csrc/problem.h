@@ -63,6 +63,15 @@ struct pasc_gb300_problem {
     int grid_sweep_max[2] = {0, 0};  // the grids the partials buffer was sized for (occupancy)
     int variant = -1;             // -1: kernel and grid chosen by timing at the first solve
     float tune_ms = 0.f;          // the chosen configuration's sweep time in the tuning runs
+    // solves that run as one cooperative launch (kernels_resident.cu): used while the kernel is
+    // left to the library (variant -1) and the state fits in shared memory
+    unsigned long long *res_slots = nullptr;
+    unsigned int res_tag = 1;     // tag of the next launch's first sweep
+    int smem_optin = 0;
+    int res_mode = -1;            // the form res_plan and the kernel attributes were made for
+    bool res_fits = false, res_refused = false;
+    pasc::ResidentPlan res_plan{};
+    bool res_used = false;        // the current solve runs that way
     cudaGraphExec_t chunk_graph = nullptr;
     int chunk_graph_len = 0, chunk_graph_variant = -1;
 
