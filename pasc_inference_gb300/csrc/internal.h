@@ -86,6 +86,41 @@ struct ResidentArgs {
     int sweeps;  // at most this many (the solve may end earlier)
 };
 
+// Device-resident state of one FP64 solve (kernels_fp64.cu).
+struct Fp64DevState {
+    double alpha, beta;     // step length of the direction at hand, its line-search step
+    double fx, fx_old;
+    double dd, dAd, gd;     // dots of the direction at hand
+    double dd_done, dAd_done;  // of the last one applied
+    double normb, coeff, eps, gamma, sigma1, sigma2;
+    double fs[MMAX_STATE];
+    int fs_last, m, maxit, coeffmode;
+    int stop_difff, stop_normgp, stop_normgp_normb, stop_Anormgp, stop_Anormgp_normb;
+    int it, hessmult, status, sweeps, error;
+};
+
+struct Fp64Plan {
+    bool ordered;         // sums in the order of the one-kernel-per-operation path
+    int blocks, threads;  // blocks 0: not used
+    int C;                // timesteps per block
+    int trees;            // of the sums
+    size_t smem;
+};
+
+struct Fp64Args {
+    double *x, *g, *d, *Ad;
+    const double *b;
+    const double *kc;  // coefficient of every cluster (theta in the penalty); null: the state's
+    Fp64DevState *st;
+    unsigned long long *slots;  // fp64_words(sms) words
+    unsigned int tag;           // the launch uses tags tag .. tag + sweeps
+    long T;
+    int C;       // timesteps per block
+    int trees;
+    int first;   // no direction yet: the first sweep evaluates the start point
+    int sweeps;
+};
+
 // Graph (R > 1) mode, mixed path (graph.cu): x and d ping-pong, buffer st->cur current.
 struct GraphSweepArgs {
     const float *data;        // T*R
@@ -245,6 +280,13 @@ bool resident_plan(int K, int mode, long T, int sms, int smem_optin, ResidentPla
 cudaError_t resident_prepare(int K, int mode, const ResidentPlan &plan);  // attributes, co-residency check
 cudaError_t launch_resident(int K, int mode, const ResidentPlan &plan, const ResidentArgs &a, cudaStream_t s);
 size_t resident_words(int sms);
+// FP64 iterations in one cooperative launch: false where they do not apply (K > 8)
+bool fp64_plan(int K, long T, int sms, Fp64Plan *p);
+size_t fp64_words(int sms);
+// x projected, g = A x - b
+cudaError_t launch_fp64_start(int K, double *x, const double *b, double *g, long T, double coeff, const double *kc,
+                              int sms, cudaStream_t s);
+cudaError_t launch_fp64_iterations(int K, const Fp64Plan &p, const Fp64Args &a, cudaStream_t s);
 cudaError_t launch_theta_f32(int K, int grid, const ThetaArgs &a, cudaStream_t s);
 cudaError_t launch_project_f32(float *x, long T, int K, cudaStream_t s);
 cudaError_t launch_matmult_f32(const float *x, float *y, long T, int K, float coeff, cudaStream_t s);

@@ -23,13 +23,10 @@
 //             to form the d of its right neighbour's first timestep, for the d'Ad pair that
 //             crosses the blocks).  It keeps x and d of these three and advances them itself;
 //             per iteration it receives their new d with the neighbours' sums.
-//   exchange  every block publishes its sums (four float-float pairs) and edge values as 64-bit
-//             words of 32 bits of payload and the sweep's tag, and polls the words of the
-//             others: a word carries its own validity, so there is no flag, fence or atomic
-//             and one L2 round trip.  Two sets of words alternate: a block publishes sweep s + 2
-//             only after it has seen every block's sweep s + 1, which those published after
-//             reading sweep s.  All blocks add the sums in the same order and apply the
-//             reference's step rules (sweep_common.cuh) to their own copy of the state.
+//   exchange  every block publishes its sums (four float-float pairs) and edge values as tagged
+//             words (grid_words.cuh) and polls the words of the others.  All blocks add the sums
+//             in the same order and apply the reference's step rules (sweep_common.cuh) to
+//             their own copy of the state.
 //
 // The launch is cooperative, so all blocks are resident while they wait for one another; every
 // wait is bounded and one that gives up sets the state's error word (PASC_ERR_TIMEOUT).
@@ -40,11 +37,11 @@
 #include "common.cuh"
 #include "project.cuh"
 #include "sweep_common.cuh"
+#include "grid_words.cuh"
 #include "internal.h"
 
 namespace pasc {
 
-constexpr unsigned int RES_WAIT_LIMIT = 1u << 22;  // polls of a word before giving up
 constexpr int RES_WORDS = 8 + 3 * KMAX_FUSED;      // words of a block's slot: sums, three edge rows
 
 // Threads of a block: up to NT that walk timesteps, and RES_MGR (the last four warps) that
@@ -70,30 +67,6 @@ struct ResSmem {
     float beta, alpha;           // of the next sweep
     int status;
 };
-
-__device__ __forceinline__ void res_store2(unsigned long long *p, unsigned long long a, unsigned long long b)
-{
-    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
-}
-__device__ __forceinline__ void res_load2(const unsigned long long *p, unsigned long long &a, unsigned long long &b)
-{
-    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
-}
-__device__ __forceinline__ void res_store(unsigned long long *p, unsigned long long a)
-{
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(a) : "memory");
-}
-__device__ __forceinline__ unsigned long long res_load(const unsigned long long *p)
-{
-    unsigned long long a;
-    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
-    return a;
-}
-__device__ __forceinline__ unsigned long long res_word(float v, unsigned int tag)
-{
-    return (unsigned long long)__float_as_uint(v) | ((unsigned long long)tag << 32);
-}
-__device__ __forceinline__ float res_payload(unsigned long long w) { return __uint_as_float((unsigned int)w); }
 
 // Addition without the renormalisation of ff_add: hi is the plain FP32 sum, lo collects its
 // exact rounding errors (Knuth's TwoSum), so hi + lo carries the precision of a float-float sum
@@ -151,11 +124,7 @@ __device__ __forceinline__ ResAhead res_look_ahead(const SpgDevState &h, int lan
         const long long k = fs_key(h.fs[q]);
         if (q != li && k > key) key = k;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const long long k = __shfl_xor_sync(0xffffffffu, key, o);
-        key = k > key ? k : key;
-    }
+    key = warp_max_key(key);
     r.fmax_other = h.m > 1 ? fs_unkey(key) : -DBL_MAX;
     // the stop tests concern the direction about to be applied (spg_finish_sweep)
     const double dfx = h.beta * h.gd + 0.5 * h.beta * h.beta * h.dAd;
@@ -591,7 +560,7 @@ __global__ void __launch_bounds__(ResShape<K>::NT + RES_MGR, 1) spg_resident_ker
             if (nb > 1 && mw == 1 && lane < 3 * K) {
                 const int which = lane / K, k = lane - which * K;
                 const int tl = which == 2 ? Cb - 1 : min(which, Cb - 1), i = tl / M;
-                res_store(slots + (size_t)blockIdx.x * RES_WORDS + 8 + lane, res_word(ds[i * S + (tl - i * M) * K + k], tag));
+                word_store(slots + (size_t)blockIdx.x * RES_WORDS + 8 + lane, word_of(ds[i * S + (tl - i * M) * K + k], tag));
             }
             __syncthreads();
             FF tot{0.f, 0.f};
@@ -602,8 +571,8 @@ __global__ void __launch_bounds__(ResShape<K>::NT + RES_MGR, 1) spg_resident_ker
                 }
                 tot = lane_sum4_ff(tot);
                 if (nb > 1 && lane < 4)
-                    res_store2(slots + (size_t)blockIdx.x * RES_WORDS + 2 * lane, res_word(tot.hi, tag),
-                               res_word(tot.lo, tag));
+                    word_store2(slots + (size_t)blockIdx.x * RES_WORDS + 2 * lane, word_of(tot.hi, tag),
+                               word_of(tot.lo, tag));
             }
             if (nb > 1) {
                 bool ok = true;
@@ -617,15 +586,15 @@ __global__ void __launch_bounds__(ResShape<K>::NT + RES_MGR, 1) spg_resident_ker
                         const int ow = 8 + (which == 0 ? 2 * K : (which - 1) * K) + k;
                         unsigned long long w = 0;
                         for (unsigned int it = 0;; it++) {
-                            w = res_load(slots + ob * RES_WORDS + ow);
-                            if ((unsigned int)(w >> 32) == tag) break;
-                            if (it >= RES_WAIT_LIMIT) {
+                            w = word_load(slots + ob * RES_WORDS + ow);
+                            if (word_valid(w, tag)) break;
+                            if (it >= WORD_WAIT_LIMIT) {
                                 ok = false;
                                 break;
                             }
                         }
-                        if (which == 0) sm.hld[k] = res_payload(w);
-                        else sm.hrd[which - 1][k] = res_payload(w);
+                        if (which == 0) sm.hld[k] = word_float(w);
+                        else sm.hrd[which - 1][k] = word_float(w);
                     }
                 }
                 // all blocks' sums: 16 bytes (a float-float pair) per load, RES_POLL loads in flight
@@ -639,22 +608,22 @@ __global__ void __launch_bounds__(ResShape<K>::NT + RES_MGR, 1) spg_resident_ker
                         for (int q = 0; q < RES_POLL; q++) {
                             const int w = w0 + q * RES_MGR;
                             if (w < 4 * nb) {
-                                res_load2(slots + (size_t)(w >> 2) * RES_WORDS + 2 * (w & 3), hi[q], lo[q]);
+                                word_load2(slots + (size_t)(w >> 2) * RES_WORDS + 2 * (w & 3), hi[q], lo[q]);
                             } else {
-                                hi[q] = lo[q] = res_word(0.f, tag);
+                                hi[q] = lo[q] = word_of(0.f, tag);
                             }
                         }
 #pragma unroll
                         for (int q = 0; q < RES_POLL; q++)
-                            all &= (unsigned int)(hi[q] >> 32) == tag && (unsigned int)(lo[q] >> 32) == tag;
+                            all &= word_valid(hi[q], tag) && word_valid(lo[q], tag);
                         if (all) break;
-                        if (it >= RES_WAIT_LIMIT) {
+                        if (it >= WORD_WAIT_LIMIT) {
                             ok = false;
                             break;
                         }
                     }
 #pragma unroll
-                    for (int q = 0; q < RES_POLL; q++) u = ff_acc(u, FF{res_payload(hi[q]), res_payload(lo[q])});
+                    for (int q = 0; q < RES_POLL; q++) u = ff_acc(u, FF{word_float(hi[q]), word_float(lo[q])});
                 }
                 u = lane_sum4_ff(u);
                 if (lane < 4) sm.red2[mw][lane] = make_float2(u.hi, u.lo);

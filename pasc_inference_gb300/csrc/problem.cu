@@ -205,7 +205,8 @@ int pasc_gb300_create(pasc_gb300_problem **out, long T, int K, int xdim, int pre
         (rc = dalloc(&p->stage64, N)) || (rc = dalloc(&p->red, dot_partials_size())) ||
         (rc = dalloc(&p->red_out, 8)) || (rc = dalloc(&p->labels_d, T)))
         return bail(rc);
-    if (cudaMallocHost((void **)&p->red_out_h, 8 * sizeof(double)) != cudaSuccess)
+    // (one page-locked block: the reductions' results and the FP64 solve's state)
+    if (cudaMallocHost((void **)&p->red_out_h, 8 * sizeof(double) + sizeof(Fp64DevState)) != cudaSuccess)
         return bail(fail(PASC_ERR_ALLOC, "create: pinned allocation failed"));
     cudaMemset(p->red, 0, dot_partials_size() * sizeof(double));
     cudaMemset(p->theta64, 0, sizeof(double) * K * xdim);
@@ -217,6 +218,15 @@ int pasc_gb300_create(pasc_gb300_problem **out, long T, int K, int xdim, int pre
             return bail(rc);
         cudaMemset(p->x, 0, sizeof(double) * N);
         cudaMemset(p->b, 0, sizeof(double) * N);
+        if (!fp64_plan(K, T, p->sms, &p->f64_plan)) {
+            p->f64_plan.blocks = 0;
+        } else {
+            const size_t nw = fp64_words(p->sms);  // the words, and the state behind them
+            if ((rc = dalloc(&p->res_slots, nw + (sizeof(Fp64DevState) + 7) / 8))) return bail(rc);
+            cudaMemset(p->res_slots, 0, nw * sizeof *p->res_slots);
+            p->st64 = reinterpret_cast<Fp64DevState *>(p->res_slots + nw);
+            p->st64_h = reinterpret_cast<Fp64DevState *>(p->red_out_h + 8);
+        }
     } else {
         // gamma and data carry zero pads (PAD_FRONT timesteps before, PAD_BACK after) so that
         // the bulk-copy sweep can copy whole tiles at the ends of the signal; the pads stay
@@ -702,9 +712,118 @@ static void fill_stats(const SpgRun &r, pasc_gb300_spgqp_stats *st)
     st->time_s = r.time_s;
 }
 
-// spgqpsolver.cpp:104-137
-static int fp64_start(pasc_gb300_problem *p)
+// ---- FP64 iterations in one cooperative launch (kernels_fp64.cu) ----
+static bool fp64_fused(const pasc_gb300_problem *p) { return p->f64_plan.blocks > 0 && !p->graph; }
+
+// n iterations while the solve runs (first: with the evaluation of the start point before them).
+// *refused: the device does not take the cooperative launch, and nothing was done.
+static int fp64_fused_run(pasc_gb300_problem *p, bool first, long n, bool *refused)
 {
+    SpgRun &r = p->run;
+    cudaStream_t s = p->stream;
+    Fp64DevState *h = p->st64_h;
+    // sweeps of one launch at most, about a tenth of a second: other work on the GPU gets its turn
+    const long most = std::max(16L, std::min(4096L, 4000000000L / std::max(1L, p->N)));
+    long left = n + (first ? 1 : 0);
+    bool begin = first;
+    do {
+        Fp64Args a;
+        a.x = p->x;
+        a.g = p->g;
+        a.d = p->d;
+        a.Ad = p->Ad;
+        a.b = p->b;
+        a.kc = p->tp ? p->tp_ck64 : nullptr;
+        a.st = p->st64;
+        a.slots = p->res_slots;
+        a.tag = p->res_tag;
+        a.T = p->T;
+        a.C = p->f64_plan.C;
+        a.trees = p->f64_plan.trees;
+        a.first = begin ? 1 : 0;
+        a.sweeps = (int)std::min(left, most);
+        const cudaError_t e = launch_fp64_iterations(p->K, p->f64_plan, a, s);
+        if (e == cudaErrorCooperativeLaunchTooLarge && begin) {
+            cudaGetLastError();
+            *refused = true;
+            return PASC_OK;
+        }
+        if (e != cudaSuccess) return fail(PASC_ERR_CUDA, "fp64 iterations: %s", cudaGetErrorString(e));
+        p->res_tag += (unsigned int)a.sweeps + 1;
+        left -= a.sweeps;
+        begin = false;
+        r.launches++;
+        CU(cudaEventRecord(p->ev1, s));
+        CU(cudaMemcpyAsync(h, p->st64, sizeof *h, cudaMemcpyDeviceToHost, s));
+        CU(cudaStreamSynchronize(s));
+    } while (left > 0 && h->status == PASC_SPG_RUNNING && !h->error);
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, p->ev0, p->ev1);
+    r.time_s += ms * 1e-3;
+    if (h->error) return fail(PASC_ERR_TIMEOUT, "fp64 iterations: a bounded wait for another block gave up");
+    r.it = h->it;
+    r.hessmult = h->hessmult;
+    r.status = h->status;
+    r.fx = h->fx;
+    r.fx_old = h->fx_old;
+    r.dd = h->dd_done;
+    r.dAd = h->dAd_done;
+    p->fx_last = r.fx;
+    p->have_fx = true;
+    return PASC_OK;
+}
+
+// the start, and the first `sweeps` iterations with it
+static int fp64_fused_start(pasc_gb300_problem *p, long sweeps, bool *refused)
+{
+    SpgRun &r = p->run;
+    const pasc_gb300_spgqp_opts *o = &r.o;
+    cudaStream_t s = p->stream;
+    CU(cudaEventRecord(p->ev0, s));
+    if (o->stop_normgp_normb || o->stop_Anormgp_normb) {  // the tests that need ||b|| (:104)
+        double v[1];
+        CU(launch_dots_f64(1, p->b, p->b, nullptr, nullptr, nullptr, nullptr, p->N, p->red, p->red_out, s));
+        r.launches++;
+        CHK(read_red(p, 1, v));
+        r.normb = sqrt(v[0]);
+    }
+    CU(launch_fp64_start(p->K, p->x, p->b, p->g, p->T, p->coeffA, p->tp ? p->tp_ck64 : nullptr, p->sms, s));  // :116-128
+    r.launches += 2;
+    Fp64DevState *h = p->st64_h;
+    memset(h, 0, sizeof *h);
+    h->alpha = o->alphainit;
+    h->fx_old = DBL_MAX;
+    h->normb = r.normb;
+    h->coeff = p->coeffA;
+    h->eps = o->eps;
+    h->gamma = o->gamma;
+    h->sigma1 = o->sigma1;
+    h->sigma2 = o->sigma2;
+    h->m = o->m;
+    h->maxit = o->maxit;
+    h->coeffmode = p->solver_type == 2 ? 1 : 0;
+    h->stop_difff = o->stop_difff;
+    h->stop_normgp = o->stop_normgp;
+    h->stop_normgp_normb = o->stop_normgp_normb;
+    h->stop_Anormgp = o->stop_Anormgp;
+    h->stop_Anormgp_normb = o->stop_Anormgp_normb;
+    h->status = PASC_SPG_RUNNING;
+    CU(cudaMemcpyAsync(p->st64, h, sizeof *h, cudaMemcpyHostToDevice, s));
+    return fp64_fused_run(p, true, sweeps, refused);
+}
+
+// spgqpsolver.cpp:104-137; the iterations that follow at once (`sweeps`) are made with it where
+// the path allows
+static int fp64_start(pasc_gb300_problem *p, long sweeps)
+{
+    if (fp64_fused(p)) {
+        bool refused = false;
+        CHK(fp64_fused_start(p, sweeps, &refused));
+        if (!refused) return PASC_OK;
+        p->f64_plan.blocks = 0;  // from here on one kernel per operation
+        p->run.launches = 0;
+        p->run.time_s = 0.0;
+    }
     SpgRun &r = p->run;
     const long N = p->N, T = p->T;
     const int K = p->K;
@@ -748,6 +867,16 @@ static int fp64_iterate(pasc_gb300_problem *p, long n)
     const int K = p->K;
     cudaStream_t s = p->stream;
     double v[3];
+    if (fp64_fused(p)) {
+        n = std::min(n, (long)o->maxit - r.it);
+        if (r.status == PASC_SPG_RUNNING && n > 0) {
+            bool refused = false;
+            CU(cudaEventRecord(p->ev0, s));
+            CHK(fp64_fused_run(p, false, n, &refused));
+        }
+        if (r.status == PASC_SPG_RUNNING && r.it >= o->maxit) r.status = PASC_SPG_MAXIT;
+        return PASC_OK;
+    }
     // SPGQPSolverC (spgqpsolver_coeff.h:611-835): d'Ad, the BB step and the A-condition without
     // the coefficient, which enters the step scalars instead
     const bool cm = p->solver_type == 2;
@@ -1298,7 +1427,7 @@ static int spgqp_start(pasc_gb300_problem *p, const pasc_gb300_spgqp_opts *o, lo
     p->run = SpgRun();
     p->run.o = *o;
     p->run.started = true;
-    return p->precision == PASC_PREC_FP64 ? fp64_start(p) : mixed_start(p, sweeps);
+    return p->precision == PASC_PREC_FP64 ? fp64_start(p, sweeps) : mixed_start(p, sweeps);
 }
 
 static int spgqp_iterate(pasc_gb300_problem *p, long n, int poll)

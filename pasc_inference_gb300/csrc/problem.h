@@ -51,6 +51,10 @@ struct pasc_gb300_problem {
     // fp64 path
     double *x = nullptr, *g = nullptr, *d = nullptr, *Ad = nullptr, *b = nullptr;
 
+    // fp64 iterations in one cooperative launch (kernels_fp64.cu); 0 blocks: one kernel per operation
+    pasc::Fp64DevState *st64 = nullptr, *st64_h = nullptr;  // behind res_slots, red_out_h
+    pasc::Fp64Plan f64_plan{};
+
     // mixed path
     float *data32 = nullptr, *theta32 = nullptr;  // data32 points past the front pad
     float *xb[2] = {nullptr, nullptr};            // past the front pad of xb_raw
@@ -65,7 +69,7 @@ struct pasc_gb300_problem {
     float tune_ms = 0.f;          // the chosen configuration's sweep time in the tuning runs
     // solves that run as one cooperative launch (kernels_resident.cu): used while the kernel is
     // left to the library (variant -1) and the state fits in shared memory
-    unsigned long long *res_slots = nullptr;
+    unsigned long long *res_slots = nullptr;  // words of the cooperative launches (both precisions)
     unsigned int res_tag = 1;     // tag of the next launch's first sweep
     int smem_optin = 0;
     int res_mode = -1;            // the form res_plan and the kernel attributes were made for
