@@ -34,33 +34,16 @@
 #include "common.cuh"
 #include "internal.h"
 #include "problem.h"
-#include "project.cuh"
+#include "project64.cuh"
+#include "adjoint.h"
 
 namespace pasc {
 
 constexpr int ADJ_NT = 256;
 constexpr int ADJ_CHUNK = 16;  // CG iterations per captured graph
 
-enum { ADJ_RUNNING = 0, ADJ_CONVERGED = 1, ADJ_MAXIT = 2, ADJ_BREAKDOWN = 4, ADJ_INNER_DONE = 8 };
-
-constexpr double ADJ_INNER_TOL = 1e-4;  // residual reduction of one FP32 refinement step
 constexpr int ADJ_MAX_OUTER = 20;
-
-struct AdjDevState {
-    double rr, rr0, pq, alpha, beta, tol;
-    double free_dims;
-    int it, maxit, status, pcur;
-    unsigned int counter;
-    double rr_in0;  // FP32 refinement: r'r at the start of the current inner solve
-    int outer;
-    unsigned int fall;  // clusters free at every timestep (their cluster-constant, zero-sum
-                        // vectors are the null space of P A P on S)
-    double nullc[8];    // component of lambda along that null space, per cluster
-    double rr64;        // FP32 refinement: FP64 r'r of the last residual
-    double rscale;      // FP32 refinement: the residual is handed to the FP32 solve times this
-                        // (its rms brought to 1: a small residual would otherwise lose its
-                        // products p'q to FP32 underflow), the correction divided by it
-};
+constexpr int ADJ_CG_ITERATIONS = 16384;  // of one cooperative launch at most
 
 struct AdjointWork {
     int K = 0, grid = 0;
@@ -70,6 +53,15 @@ struct AdjointWork {
     double *lam = nullptr, *r = nullptr, *pb[2] = {nullptr, nullptr}, *q = nullptr;  // N each
     float *r32 = nullptr, *pb32[2] = {nullptr, nullptr}, *q32 = nullptr, *d32 = nullptr;  // N each (mixed)
     cudaGraphExec_t chunk32 = nullptr;
+    // mixed: the active timesteps, their number, and the words of the cooperative solve; r32, d32
+    // and pb32[0] then hold n_active x K values
+    int *list = nullptr, *counts = nullptr, *n_h = nullptr;
+    unsigned long long *words = nullptr;
+    unsigned int tag = 1;
+    bool cg_fits = false, cg_refused = false;
+    CgPlan cg{};
+    int n_active = 0;
+    double chunk_coeff = 0.0;  // the coefficient the captured graphs were made with
     unsigned int *mask = nullptr;    // T: free clusters of each timestep (bit k)
     double *clean = nullptr, *dX = nullptr;  // T each
     double *partials = nullptr;      // grid * 16
@@ -88,7 +80,8 @@ void adjoint_free(AdjointWork *w)
     if (w->chunk) cudaGraphExecDestroy(w->chunk);
     if (w->chunk32) cudaGraphExecDestroy(w->chunk32);
     void *dev[] = {w->gam, w->gl, w->lam, w->r, w->pb[0], w->pb[1], w->q, w->mask, w->clean, w->dX,
-                   w->partials, w->out, w->st, w->ticket, w->r32, w->pb32[0], w->pb32[1], w->q32, w->d32};
+                   w->partials, w->out, w->st, w->ticket, w->r32, w->pb32[0], w->pb32[1], w->q32, w->d32,
+                   w->list, w->counts, w->words};
     for (void *p : dev)
         if (p) cudaFree(p);
     if (w->out_h) cudaFreeHost(w->out_h);
@@ -201,7 +194,7 @@ __global__ void __launch_bounds__(ADJ_NT) adj_setup_kernel(const double *gam, co
     for (int j = 0; j < 3 + K; j++) v2[j] = 0.0;
     for (long t = blockIdx.x * (long)ADJ_NT + threadIdx.x; t < T; t += (long)gridDim.x * ADJ_NT) {
         const double x = data[t];
-        double z[K], zs[K], grad[K];
+        double z[K], grad[K];
 #pragma unroll
         for (int k = 0; k < K; k++) {
             const double gc = gam[t * K + k];
@@ -220,7 +213,7 @@ __global__ void __launch_bounds__(ADJ_NT) adj_setup_kernel(const double *gam, co
 #pragma unroll
             for (int k = 0; k < K; k++) v[k] = -grad[k];
         } else {
-            project_ref_f64(z, K, zs);
+            project_f64<K>(z);
 #pragma unroll
             for (int k = 0; k < K; k++) {
                 m |= (z[k] > act_tol ? 1u : 0u) << k;
@@ -233,8 +226,10 @@ __global__ void __launch_bounds__(ADJ_NT) adj_setup_kernel(const double *gam, co
         for (int k = 0; k < K; k++) {
             r[t * K + k] = v[k];
             lam[t * K + k] = 0.0;
-            p0[t * K + k] = 0.0;
-            p1[t * K + k] = 0.0;
+            if (p0) {  // (the FP64 iterations' search directions)
+                p0[t * K + k] = 0.0;
+                p1[t * K + k] = 0.0;
+            }
             v2[0] += v[k] * v[k];
         }
         const int nf = __popc(m);
@@ -373,6 +368,21 @@ __device__ __forceinline__ void proj_free_f(float (&v)[K], unsigned int m)
     for (int k = 0; k < K; k++) v[k] = ((m >> k) & 1u) ? v[k] - mean : 0.f;
 }
 
+// the end of a residual pass: r'r = w, the outer convergence test, the inner solve's start
+__device__ __forceinline__ void adj_residual_done(AdjDevState *st, double w, double rscale)
+{
+    st->rr64 = w;
+    st->rr = w * rscale * rscale;  // r'r of the scaled FP32 residual the inner solve starts from
+    st->rr_in0 = st->rr;
+    st->beta = 0.0;
+    st->pcur = 0;
+    if (!isfinite(w)) st->status = ADJ_BREAKDOWN;
+    else if (w <= st->tol * st->tol * st->rr0) st->status = ADJ_CONVERGED;
+    else if (st->outer >= ADJ_MAX_OUTER || st->it >= st->maxit) st->status = ADJ_MAXIT;
+    else st->status = ADJ_RUNNING;
+    st->outer += 1;
+}
+
 // FP64 residual r = rhs - P A P lambda (lambda with its neighbours), rounded into r32; the
 // correction d32 and both FP32 search directions restart at 0.  Last block: r'r, the outer
 // convergence test, and the inner solve's start.
@@ -409,17 +419,58 @@ __global__ void __launch_bounds__(ADJ_NT) adj_residual_kernel(const unsigned int
     }
     double w[1];
     if (!grid_sum<1>(v, partials, &st->counter, scratch, w)) return;
-    if (threadIdx.x == 0) {
-        st->rr64 = w[0];
-        st->rr = w[0] * rscale * rscale;  // r'r of the scaled FP32 residual the inner solve starts from
-        st->rr_in0 = st->rr;
-        st->beta = 0.0;
-        st->pcur = 0;
-        if (!isfinite(w[0])) st->status = ADJ_BREAKDOWN;
-        else if (w[0] <= st->tol * st->tol * st->rr0) st->status = ADJ_CONVERGED;
-        else if (st->outer >= ADJ_MAX_OUTER || st->it >= st->maxit) st->status = ADJ_MAXIT;
-        else st->status = ADJ_RUNNING;
-        st->outer += 1;
+    if (threadIdx.x == 0) adj_residual_done(st, w[0], rscale);
+}
+
+// adj_residual_kernel over the list of active timesteps (elsewhere the residual is zero), its
+// FP32 copy in list order
+template <int K>
+__global__ void __launch_bounds__(ADJ_NT) adj_residual_list_kernel(const int *list, int n, const unsigned int *mask,
+                                                                   const double *lam, const double *rhs, float *r32,
+                                                                   long T, double coeff, double *partials,
+                                                                   AdjDevState *st)
+{
+    __shared__ double scratch[1 * (ADJ_NT / 32)];
+    const double rscale = st->rscale;
+    double v[1] = {0.0};
+    for (int e = blockIdx.x * ADJ_NT + threadIdx.x; e < n; e += gridDim.x * ADJ_NT) {
+        const long t = list[e];
+        double y[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const double lc = lam[t * K + k];
+            double ag = 0.0;
+            if (t > 0) ag += 2.0 * (lc - lam[(t - 1) * K + k]);
+            if (t < T - 1) ag += 2.0 * (lc - lam[(t + 1) * K + k]);
+            y[k] = coeff * ag;
+        }
+        proj_free<K>(y, mask[t]);
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const double rv = rhs[t * K + k] - y[k];
+            r32[(size_t)e * K + k] = (float)(rv * rscale);
+            v[0] += rv * rv;
+        }
+    }
+    double w[1];
+    if (!grid_sum<1>(v, partials, &st->counter, scratch, w)) return;
+    if (threadIdx.x == 0) adj_residual_done(st, w[0], rscale);
+}
+
+// adj_accum_kernel over the list
+template <int K>
+__global__ void __launch_bounds__(ADJ_NT) adj_accum_list_kernel(const int *list, int n, double *lam, const float *d,
+                                                                const unsigned int *mask, const AdjDevState *st)
+{
+    const double inv = 1.0 / st->rscale;
+    for (int e = blockIdx.x * ADJ_NT + threadIdx.x; e < n; e += gridDim.x * ADJ_NT) {
+        const long t = list[e];
+        double v[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] = lam[t * K + k] + (double)d[(size_t)e * K + k] * inv;
+        proj_free<K>(v, mask[t]);
+#pragma unroll
+        for (int k = 0; k < K; k++) lam[t * K + k] = v[k];
     }
 }
 
@@ -628,7 +679,7 @@ __global__ void __launch_bounds__(ADJ_NT) adj_polish_mask_kernel(const double *g
     const double a = 1.0 / (8.0 * coeff + fabs(bscale));
     for (long t = blockIdx.x * (long)ADJ_NT + threadIdx.x; t < T; t += (long)gridDim.x * ADJ_NT) {
         const double x = data[t];
-        double z[K], zs[K];
+        double z[K];
 #pragma unroll
         for (int k = 0; k < K; k++) {
             const double gc = gam[t * K + k];
@@ -638,7 +689,7 @@ __global__ void __launch_bounds__(ADJ_NT) adj_polish_mask_kernel(const double *g
             const double res = x - theta[k];
             z[k] = gc - a * (coeff * ag - bscale * res * res);
         }
-        project_ref_f64(z, K, zs);
+        project_f64<K>(z);
         unsigned int m = 0u;
 #pragma unroll
         for (int k = 0; k < K; k++) m |= (z[k] > act_tol ? 1u : 0u) << k;
@@ -823,7 +874,9 @@ static int ensure_work(pasc_gb300_problem *p)
     if (ok && p->precision == PASC_PREC_MIXED)
         ok = dal((void **)&w->gam, sizeof(double) * N) && dal((void **)&w->r32, sizeof(float) * N) &&
              dal((void **)&w->pb32[0], sizeof(float) * N) && dal((void **)&w->pb32[1], sizeof(float) * N) &&
-             dal((void **)&w->q32, sizeof(float) * N) && dal((void **)&w->d32, sizeof(float) * N);
+             dal((void **)&w->q32, sizeof(float) * N) && dal((void **)&w->d32, sizeof(float) * N) &&
+             dal((void **)&w->list, sizeof(int) * T) && dal((void **)&w->counts, sizeof(int) * cg_list_counts(T)) &&
+             dal((void **)&w->words, sizeof(unsigned long long) * cg_words(p->sms));
     if (ok) ok = cudaMallocHost((void **)&w->out_h, sizeof(double) * 16) == cudaSuccess &&
                  cudaMallocHost((void **)&w->st_h, sizeof(AdjDevState)) == cudaSuccess;
     if (!ok) {
@@ -832,6 +885,8 @@ static int ensure_work(pasc_gb300_problem *p)
     }
     cudaMemsetAsync(w->ticket, 0, sizeof(unsigned int), p->stream);
     cudaMemsetAsync(w->st, 0, sizeof(AdjDevState), p->stream);
+    if (w->words) cudaMemsetAsync(w->words, 0, sizeof(unsigned long long) * cg_words(p->sms), p->stream);
+    w->n_h = reinterpret_cast<int *>(w->out_h + 15);  // (the results take 9 of its 16 doubles)
     p->adj = w;
     return PASC_OK;
 }
@@ -848,9 +903,22 @@ static int adj_gamma(pasc_gb300_problem *p, const double **g)
     return PASC_OK;
 }
 
+// The captured graphs hold the operator's coefficient: made again when epssqr has changed.
+static void adj_drop_stale_graphs(pasc_gb300_problem *p)
+{
+    AdjointWork *w = p->adj;
+    if (w->chunk_coeff == p->coeffA) return;
+    for (cudaGraphExec_t *g : {&w->chunk, &w->chunk32}) {
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
+    w->chunk_coeff = p->coeffA;
+}
+
 static int ensure_adj_graph(pasc_gb300_problem *p)
 {
     AdjointWork *w = p->adj;
+    adj_drop_stale_graphs(p);
     if (w->chunk) return PASC_OK;
     ACU(cudaStreamSynchronize(p->stream));
     cudaGraph_t g;
@@ -879,6 +947,7 @@ static int ensure_adj_graph(pasc_gb300_problem *p)
 static int ensure_adj_graph32(pasc_gb300_problem *p)
 {
     AdjointWork *w = p->adj;
+    adj_drop_stale_graphs(p);
     if (w->chunk32) return PASC_OK;
     ACU(cudaStreamSynchronize(p->stream));
     cudaGraph_t g;
@@ -909,15 +978,30 @@ static int adj_refine(pasc_gb300_problem *p, AdjDevState *h, int *launches)
 {
     AdjointWork *w = p->adj;
     cudaStream_t s = p->stream;
+    // the active timesteps (w->mask is set); the cooperative solve where their vectors fit
+    ACU(launch_cg_list(w->mask, p->T, w->counts, w->list, s));
+    ACU(cudaMemcpyAsync(w->n_h, w->counts + cg_list_counts(p->T) - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+    ACU(cudaStreamSynchronize(s));
+    *launches += 3;
+    w->n_active = *w->n_h;
+    w->cg_fits = !w->cg_refused && cg_plan(p->K, w->n_active, p->sms, &w->cg);
+    if (!w->cg_fits) ACHK(ensure_adj_graph32(p));
+    const int list_grid = (int)std::max(1L, std::min(((long)w->n_active + ADJ_NT - 1) / ADJ_NT, (long)p->sms * 4));
     double rr_last = h->rr0;  // FP64 r'r of the last residual (the right-hand side's at first)
     auto residual = [&]() -> int {
         // scale of the next FP32 solve from the last residual: its rms about 1 (then 1e-4 after
         // each further inner solve, well inside the FP32 range)
         h->rscale = rr_last > 0.0 && isfinite(rr_last) ? 1.0 / sqrt(rr_last / (double)p->N) : 1.0;
         ACU(cudaMemcpyAsync(&w->st->rscale, &h->rscale, sizeof(double), cudaMemcpyHostToDevice, s));
-        PASC_ADJ_DISPATCH(p->K, (adj_residual_kernel<KK><<<w->grid, ADJ_NT, 0, s>>>(
-                                    w->mask, w->lam, w->r, w->r32, w->pb32[0], w->pb32[1], w->d32, p->T, p->coeffA,
-                                    w->partials, w->st)));
+        if (w->cg_fits) {
+            PASC_ADJ_DISPATCH(p->K, (adj_residual_list_kernel<KK><<<list_grid, ADJ_NT, 0, s>>>(
+                                        w->list, w->n_active, w->mask, w->lam, w->r, w->r32, p->T, p->coeffA,
+                                        w->partials, w->st)));
+        } else {
+            PASC_ADJ_DISPATCH(p->K, (adj_residual_kernel<KK><<<w->grid, ADJ_NT, 0, s>>>(
+                                        w->mask, w->lam, w->r, w->r32, w->pb32[0], w->pb32[1], w->d32, p->T, p->coeffA,
+                                        w->partials, w->st)));
+        }
         ACU(cudaGetLastError());
         *launches += 1;
         ACU(cudaMemcpyAsync(h, w->st, sizeof *h, cudaMemcpyDeviceToHost, s));
@@ -927,15 +1011,54 @@ static int adj_refine(pasc_gb300_problem *p, AdjDevState *h, int *launches)
     };
     ACHK(residual());  // lambda = 0: r32 = the right-hand side
     while (h->status == ADJ_RUNNING) {
-        while (h->status == ADJ_RUNNING) {
-            ACU(cudaGraphLaunch(w->chunk32, s));
-            *launches += 2 * ADJ_CHUNK;
+        for (bool resume = false; h->status == ADJ_RUNNING; resume = true) {
+            if (w->cg_fits) {
+                CgArgs a;
+                a.list = w->list;
+                a.mask = w->mask;
+                a.r = w->r32;
+                a.p = w->pb32[0];
+                a.d = w->d32;
+                a.st = w->st;
+                a.slots = w->words;
+                a.tag = w->tag;
+                a.T = p->T;
+                a.n = w->n_active;
+                a.C = w->cg.C;
+                a.M = w->cg.M;
+                a.iterations = ADJ_CG_ITERATIONS;
+                a.resume = resume ? 1 : 0;
+                a.coeff = (float)p->coeffA;
+                const cudaError_t e = launch_cg(p->K, w->cg, a, s);
+                if (e == cudaErrorCooperativeLaunchTooLarge && !resume) {
+                    // the device does not take the launch (an SM partition, say): all timesteps, from
+                    // the same residual
+                    cudaGetLastError();
+                    w->cg_refused = true;
+                    w->cg_fits = false;
+                    ACHK(ensure_adj_graph32(p));
+                    ACHK(residual());
+                    continue;
+                }
+                ACU(e);
+                w->tag += ADJ_CG_ITERATIONS;
+                *launches += 1;
+            } else {
+                ACU(cudaGraphLaunch(w->chunk32, s));
+                *launches += 2 * ADJ_CHUNK;
+            }
             ACU(cudaMemcpyAsync(h, w->st, sizeof *h, cudaMemcpyDeviceToHost, s));
             ACU(cudaStreamSynchronize(s));
+            if (h->timeout) return afail(PASC_ERR_TIMEOUT, "adjoint: a bounded wait for another block gave up");
         }
         if (h->status != ADJ_INNER_DONE) break;  // breakdown
-        PASC_ADJ_DISPATCH(p->K, (adj_accum_kernel<KK><<<w->grid, ADJ_NT, 0, s>>>(w->lam, w->d32, w->mask, p->T,
-                                                                                   w->st)));
+        if (w->cg_fits) {
+            PASC_ADJ_DISPATCH(p->K, (adj_accum_list_kernel<KK><<<list_grid, ADJ_NT, 0, s>>>(
+                                        w->list, w->n_active, w->lam, w->d32, w->mask, w->st)));
+        } else {
+            PASC_ADJ_DISPATCH(p->K, (adj_accum_kernel<KK><<<w->grid, ADJ_NT, 0, s>>>(w->lam, w->d32, w->mask, p->T,
+                                                                                       w->st)));
+        }
         ACU(cudaGetLastError());
         *launches += 1;
         ACHK(residual());
@@ -1000,8 +1123,7 @@ int pasc_gb300_adjoint(pasc_gb300_problem *p, const double *dloss_dgamma, const 
     const double *g = nullptr;
     ACHK(adj_gamma(p, &g));
     const bool mixed = p->precision == PASC_PREC_MIXED;
-    if (mixed) ACHK(ensure_adj_graph32(p));
-    else ACHK(ensure_adj_graph(p));
+    if (!mixed) ACHK(ensure_adj_graph(p));
     ACU(cudaEventRecord(p->ev0, s));
 
     AdjDevState *h = w->st_h;
@@ -1011,7 +1133,8 @@ int pasc_gb300_adjoint(pasc_gb300_problem *p, const double *dloss_dgamma, const 
     ACU(cudaMemcpyAsync(w->st, h, sizeof *h, cudaMemcpyHostToDevice, s));
     PASC_ADJ_DISPATCH(p->K, (adj_setup_kernel<KK><<<w->grid, ADJ_NT, 0, s>>>(
                                 g, w->gl, p->data64, p->theta64, p->T, p->coeffA, p->coeffB, o->act_tol,
-                                w->mask, w->lam, w->r, w->pb[0], w->pb[1], w->partials, w->st)));
+                                w->mask, w->lam, w->r, mixed ? nullptr : w->pb[0], mixed ? nullptr : w->pb[1],
+                                w->partials, w->st)));
     ACU(cudaGetLastError());
     int launches = 1;
     ACU(cudaMemcpyAsync(h, w->st, sizeof *h, cudaMemcpyDeviceToHost, s));
@@ -1092,8 +1215,7 @@ int pasc_gb300_polish(pasc_gb300_problem *p, const pasc_gb300_polish_opts *o, pa
     double *gam = mixed ? w->gam : p->x;
     double *backup = w->gl;  // gamma at the start of a round (a kept dloss/dgamma is dropped anyway)
     if (mixed) ACU(launch_f32_to_f64(p->xb[p->cur], gam, p->N, s));
-    if (mixed) ACHK(ensure_adj_graph32(p));
-    else ACHK(ensure_adj_graph(p));
+    if (!mixed) ACHK(ensure_adj_graph(p));
     ACU(cudaEventRecord(p->ev0, s));
     AdjDevState *h = w->st_h;
     int launches = mixed ? 1 : 0, rounds = 0, cg_it = 0, cg_status = 0;
@@ -1135,7 +1257,8 @@ int pasc_gb300_polish(pasc_gb300_problem *p, const pasc_gb300_polish_opts *o, pa
         launches += 2;
         PASC_ADJ_DISPATCH(p->K, (adj_setup_kernel<KK, true><<<w->grid, ADJ_NT, 0, s>>>(
                                     gam, nullptr, p->data64, p->theta64, p->T, p->coeffA, p->coeffB, o->act_tol,
-                                    w->mask, w->lam, w->r, w->pb[0], w->pb[1], w->partials, w->st)));
+                                    w->mask, w->lam, w->r, mixed ? nullptr : w->pb[0], mixed ? nullptr : w->pb[1],
+                                    w->partials, w->st)));
         ACU(cudaGetLastError());
         launches++;
         ACU(cudaMemcpyAsync(h, w->st, sizeof *h, cudaMemcpyDeviceToHost, s));

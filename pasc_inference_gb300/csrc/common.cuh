@@ -90,6 +90,23 @@ __device__ __forceinline__ FF ff_add(FF a, FF b)
     return FF{hi, __fsub_rn(e, __fsub_rn(hi, s))};
 }
 
+// Addition without the renormalisation of ff_add: hi is the plain FP32 sum, lo collects its
+// exact rounding errors (Knuth's TwoSum), so hi + lo carries the precision of a float-float sum
+// while a chain of additions waits for one FP32 addition per link instead of eleven.
+__device__ __forceinline__ FF ff_acc(FF a, FF b)
+{
+    const float s = __fadd_rn(a.hi, b.hi);
+    const float bv = __fsub_rn(s, a.hi);
+    const float av = __fsub_rn(s, bv);
+    const float e = __fadd_rn(__fsub_rn(a.hi, av), __fsub_rn(b.hi, bv));
+    return FF{s, __fadd_rn(__fadd_rn(a.lo, b.lo), e)};
+}
+
+__device__ __forceinline__ FF ff_shfl_xor(FF a, int m)
+{
+    return FF{__shfl_xor_sync(0xffffffffu, a.hi, m), __shfl_xor_sync(0xffffffffu, a.lo, m)};
+}
+
 __device__ __forceinline__ double ff_value(FF a) { return (double)a.hi + (double)a.lo; }
 
 template <int NV>

@@ -68,23 +68,6 @@ struct ResSmem {
     int status;
 };
 
-// Addition without the renormalisation of ff_add: hi is the plain FP32 sum, lo collects its
-// exact rounding errors (Knuth's TwoSum), so hi + lo carries the precision of a float-float sum
-// while a chain of additions waits for one FP32 addition per link instead of eleven.
-__device__ __forceinline__ FF ff_acc(FF a, FF b)
-{
-    const float s = __fadd_rn(a.hi, b.hi);
-    const float bv = __fsub_rn(s, a.hi);
-    const float av = __fsub_rn(s, bv);
-    const float e = __fadd_rn(__fsub_rn(a.hi, av), __fsub_rn(b.hi, bv));
-    return FF{s, __fadd_rn(__fadd_rn(a.lo, b.lo), e)};
-}
-
-__device__ __forceinline__ FF ff_shfl_xor(FF a, int m)
-{
-    return FF{__shfl_xor_sync(0xffffffffu, a.hi, m), __shfl_xor_sync(0xffffffffu, a.lo, m)};
-}
-
 // Lanes hold partial sums of value lane & 3: sums over the lanes of each value.
 __device__ __forceinline__ FF lane_sum4_ff(FF r)
 {
