@@ -153,13 +153,12 @@ __device__ __forceinline__ void block_sum_ff(FF (&v)[NV], float2 *scratch)
 // loads a thread issues before adding them (the additions stay in slot order, so the sums do
 // not depend on it): one L2 latency per BATCH slots, for kernels with registers to spare.
 template <int BATCH = 1>
-__device__ __forceinline__ bool sweep_grid_sum4(const KahanF &f, float dd, float dAd, float gd, float2 *partials,
+__device__ __forceinline__ bool sweep_grid_sum4(FF (&v)[4], float2 *partials,
                                                long slot, unsigned int *ticket, unsigned int nslot, long slot0,
                                                long stride, float2 *scratch, double (&w)[4],
                                                const void *snap_src = nullptr, void *snap_dst = nullptr,
                                                int snap_bytes = 0)
 {
-    FF v[4] = {FF{f.s, f.c}, ff_make(dd), ff_make(dAd), ff_make(gd)};
     block_sum_ff<4>(v, scratch);
     if (threadIdx.x == 0) {
 #pragma unroll
@@ -209,6 +208,18 @@ __device__ __forceinline__ bool sweep_grid_sum4(const KahanF &f, float dd, float
 #pragma unroll
     for (int q = 0; q < 4; q++) w[q] = ff_value(u[q]);
     return true;
+}
+
+template <int BATCH = 1>
+__device__ __forceinline__ bool sweep_grid_sum4(const KahanF &f, float dd, float dAd, float gd, float2 *partials,
+                                               long slot, unsigned int *ticket, unsigned int nslot, long slot0,
+                                               long stride, float2 *scratch, double (&w)[4],
+                                               const void *snap_src = nullptr, void *snap_dst = nullptr,
+                                               int snap_bytes = 0)
+{
+    FF v[4] = {FF{f.s, f.c}, ff_make(dd), ff_make(dAd), ff_make(gd)};
+    return sweep_grid_sum4<BATCH>(v, partials, slot, ticket, nslot, slot0, stride, scratch, w, snap_src, snap_dst,
+                                  snap_bytes);
 }
 
 // Last-block-done ticket: returns true in every thread of the block that finished last.

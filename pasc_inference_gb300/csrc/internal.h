@@ -138,9 +138,11 @@ struct ImageSweepArgs {
     const float *data;        // W*H, row-major
     const float *theta;       // K
     float *xb0, *xb1;         // gamma, ping-pong (buffer st->cur current)
+    float *db0, *db1;         // direction d of the current gamma
     double *partials;         // gridDim.x * 4
     SpgDevState *st;
     int W, H;
+    int th;                   // owned rows of a strip tile
 };
 
 struct ThetaArgs {
@@ -244,8 +246,7 @@ cudaError_t launch_graph_matmult_f64(const double *x, double *y, long T, long R,
                                      const int *ptr, const int *idx, cudaStream_t s, const double *kc = nullptr);
 
 bool graph_is_grid2d(long R, const int *ptr, const int *idx, int *W, int *H);  // host check
-int image_sweep_blocks_per_sm(int K);  // also sets the kernels' shared-memory limit
-int image_sweep_tiles(int W, int H);
+void image_sweep_plan(int K, int W, int H, int sms, int *th, int *blocks);
 cudaError_t launch_image_sweep(int K, bool init, int grid, const ImageSweepArgs &a, cudaStream_t s);
 
 int batch_tile_width();

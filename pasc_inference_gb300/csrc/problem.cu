@@ -1010,8 +1010,11 @@ static cudaError_t launch_variant(pasc_gb300_problem *p, int v, bool init, const
         g.xb1 = p->xb[1];
         g.partials = p->gpartials;
         g.st = p->st;
+        g.db0 = p->db_raw[0];
+        g.db1 = p->db_raw[1];
         g.W = p->img_W;
         g.H = p->img_H;
+        g.th = p->img_th;
         return launch_image_sweep(p->K, init, p->grid_image, g, p->stream);
     }
     if (p->graph) {
@@ -1898,11 +1901,9 @@ int pasc_gb300_create_graph(pasc_gb300_problem **out, long T, long R, int K, int
         p->grid_graph = graph_sweep_grid(T * R);
         int W = 0, H = 0;
         if (T == 1 && graph_is_grid2d(R, nbr_ptr, nbr_idx, &W, &H)) {
-            const int per_sm = image_sweep_blocks_per_sm(K);
-            const int tiles = image_sweep_tiles(W, H);
             p->img_W = W;
             p->img_H = H;
-            p->grid_image = std::max(1, std::min(tiles, per_sm * p->sms));
+            image_sweep_plan(K, W, H, p->sms, &p->img_th, &p->grid_image);
         }
         const int gp = std::max(p->grid_graph, p->grid_image);
         if ((rc = dalloc(&p->db_raw[0], N)) || (rc = dalloc(&p->db_raw[1], N)) ||
