@@ -98,6 +98,110 @@ __global__ void fem_prolongate_kernel(const TIn *g2, TOut *g1, long T1, long T2,
     g1[idx] = (TOut)v;
 }
 
+// ---- FEM-SUM of the mixed path ----
+// lo[j]: the first fine timestep of coarse timestep j (lo[T2] = T1), computed once when the
+// reduction is set up: the FP64 rounding of the reference's expressions costs as much as the sums.
+// The fine field is read, and the prolongated one written, in consecutive order.  Sums: gamma, an
+// FP32 field, float-float; the residual in FP64 with three instead of 3K operations per fine
+// timestep,
+//     sum (x_t - theta_k)^2 = S2 - 2 e S1 + n e^2,   S1 = sum (x_t - c), S2 = sum (x_t - c)^2, e = theta_k - c
+// with c the block's first value, so that the cancellation is bounded by the spread of the
+// values themselves; the result is rounded to FP32 either way.  (One thread per coarse entry,
+// summing in FP64 with a stride of K: 95 us for both reductions at T = 2e6, K = 3, T2 = T/10; here
+// 24 and 12, and the copy back 15.)
+constexpr int FEM_NT = 256;
+
+__global__ void __launch_bounds__(FEM_NT) fem_bounds_kernel(int *lo, long T2, double diff)
+{
+    const long j = (long)blockIdx.x * FEM_NT + threadIdx.x;
+    if (j <= T2) lo[j] = (int)(long)round(fem_mul(j, diff));
+}
+
+__global__ void __launch_bounds__(FEM_NT) fem_sum_field_kernel(const float *__restrict__ g1, float *__restrict__ g2,
+                                                               const int *__restrict__ lo, unsigned int n, int K, double scale)
+{
+    const unsigned int e = blockIdx.x * FEM_NT + threadIdx.x;
+    if (e >= n) return;
+    const unsigned int j = e / (unsigned int)K;
+    const int k = (int)(e - j * K);
+    const int hi = lo[j + 1];
+    FF s{0.f, 0.f};
+#pragma unroll 4
+    for (int i = lo[j]; i < hi; i++) s = ff_acc(s, ff_make(__ldg(g1 + (long)i * K + k)));
+    g2[e] = scale == 1.0 ? s.hi + s.lo : (float)__dmul_rn(ff_value(s), scale);
+}
+
+template <int K>
+__global__ void __launch_bounds__(FEM_NT) fem_sum_residual_kernel(const double *__restrict__ data,
+                                                                  const double *__restrict__ theta, float *__restrict__ g2,
+                                                                  const int *__restrict__ lo, int T2, double scale)
+{
+    const int j = blockIdx.x * FEM_NT + threadIdx.x;
+    if (j >= T2) return;
+    const int a = lo[j], b = lo[j + 1];
+    const double c = a < b ? data[a] : 0.0;
+    double u = 0.0, v = 0.0;
+#pragma unroll 4
+    for (int i = a; i < b; i++) {
+        const double d = data[i] - c;
+        u += d;
+        v = fma(d, d, v);
+    }
+    const double n = (double)(b - a), u2 = -2.0 * u;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const double d = theta[k] - c;
+        g2[(long)j * K + k] = (float)(fma(d, fma(n, d, u2), v) * scale);
+    }
+}
+
+__global__ void __launch_bounds__(FEM_NT) fem_copy_kernel(const float *__restrict__ g2, float *__restrict__ g1,
+                                                          const int *__restrict__ lo, int T1, int T2, int K, double inv)
+{
+    const int t = blockIdx.x * FEM_NT + threadIdx.x;
+    if (t >= T1) return;
+    int j = (int)((double)t * inv);  // a guess, corrected by the bounds
+    j = j < T2 ? j : T2 - 1;
+    while (j > 0 && t < __ldg(lo + j)) j--;
+    while (j < T2 - 1 && t >= __ldg(lo + j + 1)) j++;
+    for (int k = 0; k < K; k++) g1[(long)t * K + k] = __ldg(g2 + (long)j * K + k);
+}
+
+cudaError_t launch_fem_bounds(int *lo, long T1, long T2, cudaStream_t s)
+{
+    fem_bounds_kernel<<<(unsigned int)(T2 / FEM_NT + 1), FEM_NT, 0, s>>>(lo, T2, (double)T1 / (double)T2);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fem_sum_field(const float *g1, float *g2, const int *lo, long T2, int K, double scale, cudaStream_t s)
+{
+    const long n = T2 * K;
+    fem_sum_field_kernel<<<(unsigned int)((n + FEM_NT - 1) / FEM_NT), FEM_NT, 0, s>>>(g1, g2, lo, (unsigned int)n, K, scale);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fem_sum_residual(const double *data, const double *theta, float *g2, const int *lo, long T2, int K,
+                                    double scale, cudaStream_t s)
+{
+    const unsigned int grid = (unsigned int)((T2 + FEM_NT - 1) / FEM_NT);
+    switch (K) {
+#define PASC_CASE(KK) \
+    case KK: fem_sum_residual_kernel<KK><<<grid, FEM_NT, 0, s>>>(data, theta, g2, lo, (int)T2, scale); break;
+        PASC_CASE(1) PASC_CASE(2) PASC_CASE(3) PASC_CASE(4)
+        PASC_CASE(5) PASC_CASE(6) PASC_CASE(7) PASC_CASE(8)
+#undef PASC_CASE
+        default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fem_copy(const float *g2, float *g1, const int *lo, long T1, long T2, int K, cudaStream_t s)
+{
+    fem_copy_kernel<<<(unsigned int)((T1 + FEM_NT - 1) / FEM_NT), FEM_NT, 0, s>>>(g2, g1, lo, (int)T1, (int)T2, K,
+                                                                                 (double)T2 / (double)T1);
+    return cudaGetLastError();
+}
+
 static double fem_diff(long T1, long T2, int type)
 {
     return type == 0 ? (double)T1 / (double)T2 : (double)(T1 - 1) / (double)(T2 - 1);

@@ -238,6 +238,14 @@ cudaError_t launch_fem_reduce(const TIn *g1, const double *data, const double *t
 template <typename TIn, typename TOut>
 cudaError_t launch_fem_prolongate(const TIn *g2, TOut *g1, long T1, long T2, int K, int type, cudaStream_t s);
 
+// FEM-SUM of the mixed path: bounds of the coarse timesteps (T2 + 1 ints), made once; the field's
+// sums (times scale), the residual's, and the copy back
+cudaError_t launch_fem_bounds(int *lo, long T1, long T2, cudaStream_t s);
+cudaError_t launch_fem_sum_field(const float *g1, float *g2, const int *lo, long T2, int K, double scale, cudaStream_t s);
+cudaError_t launch_fem_sum_residual(const double *data, const double *theta, float *g2, const int *lo, long T2, int K,
+                                    double scale, cudaStream_t s);
+cudaError_t launch_fem_copy(const float *g2, float *g1, const int *lo, long T1, long T2, int K, cudaStream_t s);
+
 // Graph (R > 1) and image mode (graph.cu).
 const char *graph_check(long R, const int *ptr, const int *idx);  // null: valid
 int graph_sweep_grid(long nblocks);

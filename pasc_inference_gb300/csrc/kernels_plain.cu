@@ -181,18 +181,48 @@ __global__ void permute_kernel(const F *src, F *dst, long T, int K, long R)
     }
 }
 
-cudaError_t launch_permute_f64(const double *src, double *dst, long T, int K, cudaStream_t s, long R)
+// the same for R = 1 and few clusters, one thread per timestep: no division by K per value, reads and
+// writes consecutive over the threads
+template <typename F, int K>
+__global__ void __launch_bounds__(PLAIN_NT) permute_chain_kernel(const F *__restrict__ src, F *__restrict__ dst, long T)
+{
+    const long stride = (long)gridDim.x * PLAIN_NT;
+    for (long t = (long)blockIdx.x * PLAIN_NT + threadIdx.x; t < T; t += stride) {
+        F v[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] = src[(long)k * T + t];
+#pragma unroll
+        for (int k = 0; k < K; k++) dst[t * K + k] = v[k];
+    }
+}
+
+// (T = 2e6, K = 3, FP32: 25 us by permute_kernel, 11 by permute_chain_kernel)
+template <typename F>
+static cudaError_t launch_permute(const F *src, F *dst, long T, int K, cudaStream_t s, long R)
 {
     if (T <= 0) return cudaSuccess;
-    permute_kernel<double><<<grid_elems(T * K), PLAIN_NT, 0, s>>>(src, dst, T, K, R);
+    if (R == 1 && K <= 8) {
+        const int g = grid_elems(T);
+        switch (K) {
+#define PASC_CASE(KK) case KK: permute_chain_kernel<F, KK><<<g, PLAIN_NT, 0, s>>>(src, dst, T); break;
+            PASC_CASE(1) PASC_CASE(2) PASC_CASE(3) PASC_CASE(4)
+            PASC_CASE(5) PASC_CASE(6) PASC_CASE(7) PASC_CASE(8)
+#undef PASC_CASE
+        }
+        return cudaGetLastError();
+    }
+    permute_kernel<F><<<grid_elems(T * K), PLAIN_NT, 0, s>>>(src, dst, T, K, R);
     return cudaGetLastError();
+}
+
+cudaError_t launch_permute_f64(const double *src, double *dst, long T, int K, cudaStream_t s, long R)
+{
+    return launch_permute(src, dst, T, K, s, R);
 }
 
 cudaError_t launch_permute_f32(const float *src, float *dst, long T, int K, cudaStream_t s, long R)
 {
-    if (T <= 0) return cudaSuccess;
-    permute_kernel<float><<<grid_elems(T * K), PLAIN_NT, 0, s>>>(src, dst, T, K, R);
-    return cudaGetLastError();
+    return launch_permute(src, dst, T, K, s, R);
 }
 
 // ---------------------------------------------------------------------------------------

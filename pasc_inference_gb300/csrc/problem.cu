@@ -68,7 +68,7 @@ static void free_all(pasc_gb300_problem *p)
                    p->d, p->Ad, p->b, p->data32_raw, p->theta32, p->xb_raw[0], p->xb_raw[1], p->st,
                    p->partials, p->xbf, p->xnorm, p->bmat_raw, p->theta_split, p->theta_f32, p->tnorm,
                    p->mc_partials, p->mc_err, p->tp_ck64, p->tp_kw32, p->gptr, p->gidx, p->db_raw[0],
-                   p->db_raw[1], p->gpartials, p->stage32, p->res_slots};
+                   p->db_raw[1], p->gpartials, p->stage32, p->res_slots, p->fem_lo};
     for (void *q : dev)
         if (q) cudaFree(q);
     if (p->st_h) cudaFreeHost(p->st_h);
@@ -407,15 +407,20 @@ static int fem_update_b_async(pasc_gb300_problem *p, int *launches)
         CU((launch_fem_reduce<double, double>(nullptr, p->data64, p->theta64, q->b, T, T2, K, type, q->coeffB, s)));
         CU((launch_fem_reduce<double, double>(p->x, nullptr, nullptr, q->x, T, T2, K, type, 1.0, s)));
     } else {
+        const bool sum = p->fem_lo != nullptr;  // FEM-SUM
         if (p->xdim > 1) {
             // the full b = bscale ||X_t - theta_k||^2 (FP32), then its reduction rescaled
             CHK(mc_residual_async(p, launches));
-            CU((launch_fem_reduce<float, float>(p->bmat, nullptr, nullptr, q->bmat, T, T2, K, type,
-                                               q->coeffB / p->coeffB, s)));
+            const double sc = q->coeffB / p->coeffB;
+            if (sum) CU(launch_fem_sum_field(p->bmat, q->bmat, p->fem_lo, T2, K, sc, s));
+            else CU((launch_fem_reduce<float, float>(p->bmat, nullptr, nullptr, q->bmat, T, T2, K, type, sc, s)));
+        } else if (sum) {
+            CU(launch_fem_sum_residual(p->data64, p->theta64, q->bmat, p->fem_lo, T2, K, q->coeffB, s));
         } else {
             CU((launch_fem_reduce<float, float>(nullptr, p->data64, p->theta64, q->bmat, T, T2, K, type, q->coeffB, s)));
         }
-        CU((launch_fem_reduce<float, float>(p->xb[p->cur], nullptr, nullptr, q->xb[q->cur], T, T2, K, type, 1.0, s)));
+        if (sum) CU(launch_fem_sum_field(p->xb[p->cur], q->xb[q->cur], p->fem_lo, T2, K, 1.0, s));
+        else CU((launch_fem_reduce<float, float>(p->xb[p->cur], nullptr, nullptr, q->xb[q->cur], T, T2, K, type, 1.0, s)));
     }
     if (launches) *launches += 2;
     // the inner handle works on its own stream: its solve must see the reduced b and x
@@ -1480,6 +1485,8 @@ int pasc_gb300_spgqp_solve(pasc_gb300_problem *p, const pasc_gb300_spgqp_opts *o
         CHK(pasc_gb300_spgqp_solve(q, o, &ist));
         if (p->precision == PASC_PREC_FP64)
             CU((launch_fem_prolongate<double, double>(q->x, p->x, p->T, q->T, p->K, p->fem_type, p->stream)));
+        else if (p->fem_lo)
+            CU(launch_fem_copy(q->xb[q->cur], p->xb[p->cur], p->fem_lo, p->T, q->T, p->K, p->stream));
         else
             CU((launch_fem_prolongate<float, float>(q->xb[q->cur], p->xb[p->cur], p->T, q->T, p->K, p->fem_type,
                                                    p->stream)));
@@ -1698,6 +1705,8 @@ int pasc_gb300_set_fem(pasc_gb300_problem *p, double fem_reduce, int fem_type)
         free_all(p->fem_inner);
         p->fem_inner = nullptr;
     }
+    if (p->fem_lo) cudaFree(p->fem_lo);
+    p->fem_lo = nullptr;
     p->fem_reduce = fem_reduce;
     p->fem_type = fem_type;
     p->run.started = false;
@@ -1724,6 +1733,13 @@ int pasc_gb300_set_fem(pasc_gb300_problem *p, double fem_reduce, int fem_type)
         q->grid_sweep_max[1] = q->grid_sweep[1];
         g = (long)sweep_tma_blocks_per_sm(p->K, true, true) * q->sms;
         q->grid_sweep_init[1] = (int)(g < nt_tma ? (g < 1 ? 1 : g) : nt_tma);
+    }
+    if (p->precision == PASC_PREC_MIXED && fem_type == 0) {
+        const int rc = dalloc(&p->fem_lo, (size_t)T2 + 1);
+        if (rc || launch_fem_bounds(p->fem_lo, p->T, T2, p->stream) != cudaSuccess) {
+            free_all(q);
+            return rc ? rc : fail(PASC_ERR_CUDA, "set_fem: kernel launch failed");
+        }
     }
     q->solver_type = p->solver_type;
     p->fem_inner = q;

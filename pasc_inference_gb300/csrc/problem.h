@@ -105,6 +105,7 @@ struct pasc_gb300_problem {
     double fem_reduce = 1.0;
     int fem_type = 0;
     pasc_gb300_problem *fem_inner = nullptr;
+    int *fem_lo = nullptr;                 // mixed FEM-SUM: bounds of the coarse timesteps
     bool b_external = false;               // inner handle: b is written by the owner
 
     // graph (R > 1) / image mode (pasc_gb300_create_graph): T above counts the T*R blocks of K;
