@@ -75,6 +75,8 @@ static void free_all(pasc_gb300_problem *p)
     if (p->red_out_h) cudaFreeHost(p->red_out_h);
     if (p->ev0) cudaEventDestroy(p->ev0);
     if (p->ev1) cudaEventDestroy(p->ev1);
+    for (cudaEvent_t e : p->ev_poll)
+        if (e) cudaEventDestroy(e);
     if (p->stream) cudaStreamDestroy(p->stream);
     delete p;
 }
@@ -242,9 +244,9 @@ int pasc_gb300_create(pasc_gb300_problem **out, long T, int K, int xdim, int pre
         p->xb[0] = p->xb_raw[0] + (size_t)PAD_FRONT * K;
         p->xb[1] = p->xb_raw[1] + (size_t)PAD_FRONT * K;
         p->data32 = p->data32_raw + PAD_FRONT;
-        if (cudaMallocHost((void **)&p->st_h, sizeof(SpgDevState)) != cudaSuccess)
+        if (cudaMallocHost((void **)&p->st_h, 3 * sizeof(SpgDevState)) != cudaSuccess)
             return bail(fail(PASC_ERR_ALLOC, "create: pinned allocation failed"));
-        memset(p->st_h, 0, sizeof(SpgDevState));
+        memset(p->st_h, 0, 3 * sizeof(SpgDevState));
         cudaMemset(p->st, 0, sizeof(SpgDevState));
         cudaMemset(p->theta32, 0, sizeof(float) * K);
         auto grid = [&](long per_sm, long ntiles) {
@@ -1343,6 +1345,7 @@ static int mixed_start(pasc_gb300_problem *p, long sweeps)
     if (o->stop_normgp_normb || o->stop_Anormgp_normb)
         return fail(PASC_ERR_NOTSUPP, "spgqp: ||b||-scaled stopping tests need the fp64 path");
     cudaStream_t s = p->stream;
+    p->start_in_flight = false;
     CHK(resident_choose(p));
     if (p->res_used) CHK(resident_run(p, true, sweeps));
     if (p->res_used) return PASC_OK;
@@ -1355,27 +1358,34 @@ static int mixed_start(pasc_gb300_problem *p, long sweeps)
     CU(cudaEventRecord(p->ev0, s));
     CU(cudaMemcpyAsync(p->st, h, sizeof(SpgDevState), cudaMemcpyHostToDevice, s));
     CU(launch_variant(p, p->variant, true, a));
+    p->run.launches += p->graph && p->variant == 0 ? 2 : 1;
+    if (sweeps > 0) {  // the iterations follow at once: the state is read after them
+        p->start_in_flight = true;
+        p->run.hessmult = 1;
+        p->run.status = PASC_SPG_RUNNING;
+        return PASC_OK;
+    }
     CU(cudaEventRecord(p->ev1, s));
     CU(cudaMemcpyAsync(h, p->st, sizeof(SpgDevState), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, p->ev0, p->ev1);
-    p->run.launches += p->graph && p->variant == 0 ? 2 : 1;
     p->run.time_s += ms * 1e-3;
     CHK(check_device_error(p));
     sync_run_from_device(p);
     return PASC_OK;
 }
 
-// Launches n regular sweeps.  With poll, the status word is read after chunks of growing
-// length and launching stops once the solve has ended; without poll exactly n sweeps are
-// launched back to back (sweeps after the end return at once) and timed as one region.
+// Launches n regular sweeps.  With poll, the status is read after chunks of growing length, while
+// the next chunk runs (a chunk launched after the end returns at once, about 1.5 us per sweep, where
+// waiting for the status before each launch left the GPU idle for about 12 us); launching stops
+// once a status read says that the solve has ended.  Without poll exactly n sweeps are launched
+// back to back (sweeps after the end return at once) and timed as one region.
 static int mixed_iterate(pasc_gb300_problem *p, long n, int poll)
 {
     cudaStream_t s = p->stream;
-    SweepArgs a;
-    sweep_args(p, &a);
-    SpgDevState *h = p->st_h;
+    const bool started = p->start_in_flight;
+    p->start_in_flight = false;
     if (p->run.status != PASC_SPG_RUNNING) return PASC_OK;
     const long room = p->run.o.maxit - p->run.it;
     if (n > room) n = room;
@@ -1385,11 +1395,16 @@ static int mixed_iterate(pasc_gb300_problem *p, long n, int poll)
         if (p->run.status == PASC_SPG_RUNNING && p->run.it >= p->run.o.maxit) p->run.status = PASC_SPG_MAXIT;
         return PASC_OK;
     }
+    SweepArgs a;
+    sweep_args(p, &a);
+    SpgDevState *h = p->st_h;
     CHK(ensure_chunk_graph(p));
+    for (cudaEvent_t &e : p->ev_poll)
+        if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     long done = 0;
-    int step = 0;
+    int step = 0, last = -1;  // last: the poll in flight
     const int sched[] = {2, 4, 8};
-    CU(cudaEventRecord(p->ev0, s));
+    if (!started) CU(cudaEventRecord(p->ev0, s));
     while (done < n) {
         long want = poll ? (step < 3 ? sched[step] : GRAPH_CHUNK) : GRAPH_CHUNK;
         step++;
@@ -1401,10 +1416,15 @@ static int mixed_iterate(pasc_gb300_problem *p, long n, int poll)
         }
         done += want;
         p->run.launches += (int)want * (p->graph && p->variant == 0 ? 2 : 1);
-        if (poll) {
-            CU(cudaMemcpyAsync(h, p->st, sizeof(SpgDevState), cudaMemcpyDeviceToHost, s));
-            CU(cudaStreamSynchronize(s));
-            if (h->status != PASC_SPG_RUNNING || h->error) break;
+        if (poll && done < n) {
+            const int slot = last == 0 ? 1 : 0;
+            CU(cudaMemcpyAsync(h + 1 + slot, p->st, sizeof(SpgDevState), cudaMemcpyDeviceToHost, s));
+            CU(cudaEventRecord(p->ev_poll[slot], s));
+            if (last >= 0) {
+                CU(cudaEventSynchronize(p->ev_poll[last]));
+                if (h[1 + last].status != PASC_SPG_RUNNING || h[1 + last].error) break;
+            }
+            last = slot;
         }
     }
     CU(cudaEventRecord(p->ev1, s));

@@ -59,7 +59,9 @@ struct pasc_gb300_problem {
     float *data32 = nullptr, *theta32 = nullptr;  // data32 points past the front pad
     float *xb[2] = {nullptr, nullptr};            // past the front pad of xb_raw
     float *xb_raw[2] = {nullptr, nullptr}, *data32_raw = nullptr;
-    pasc::SpgDevState *st = nullptr, *st_h = nullptr;
+    pasc::SpgDevState *st = nullptr, *st_h = nullptr;  // st_h: three mirrors (the state, two polls in flight)
+    cudaEvent_t ev_poll[2] = {nullptr, nullptr};
+    bool start_in_flight = false;  // the INIT sweep was launched by a solve that iterates at once: not read back yet
     double *partials = nullptr;
     int cur = 0;
     // sweep kernels: 0 = one timestep per thread, 1 = bulk-copy tiles, 4 timesteps per thread
