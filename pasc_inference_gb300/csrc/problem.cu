@@ -220,15 +220,6 @@ int pasc_gb300_create(pasc_gb300_problem **out, long T, int K, int xdim, int pre
             return bail(rc);
         cudaMemset(p->x, 0, sizeof(double) * N);
         cudaMemset(p->b, 0, sizeof(double) * N);
-        if (!fp64_plan(K, T, p->sms, &p->f64_plan)) {
-            p->f64_plan.blocks = 0;
-        } else {
-            const size_t nw = fp64_words(p->sms);  // the words, and the state behind them
-            if ((rc = dalloc(&p->res_slots, nw + (sizeof(Fp64DevState) + 7) / 8))) return bail(rc);
-            cudaMemset(p->res_slots, 0, nw * sizeof *p->res_slots);
-            p->st64 = reinterpret_cast<Fp64DevState *>(p->res_slots + nw);
-            p->st64_h = reinterpret_cast<Fp64DevState *>(p->red_out_h + 8);
-        }
     } else {
         // gamma and data carry zero pads (PAD_FRONT timesteps before, PAD_BACK after) so that
         // the bulk-copy sweep can copy whole tiles at the ends of the signal; the pads stay
@@ -720,7 +711,28 @@ static void fill_stats(const SpgRun &r, pasc_gb300_spgqp_stats *st)
 }
 
 // ---- FP64 iterations in one cooperative launch (kernels_fp64.cu) ----
-static bool fp64_fused(const pasc_gb300_problem *p) { return p->f64_plan.blocks > 0 && !p->graph; }
+static bool fp64_fused(const pasc_gb300_problem *p) { return p->f64_plan.blocks > 0; }
+
+// the plan and its buffers, at the first solve
+static int fp64_prepare(pasc_gb300_problem *p)
+{
+    if (p->f64_planned) return PASC_OK;
+    p->f64_planned = true;
+    p->f64_plan.blocks = 0;
+    Fp64Plan plan;
+    if (p->graph || !fp64_plan(p->K, p->T, p->sms, &plan)) return PASC_OK;
+    const size_t nw = fp64_words(p->sms);  // the words, and the state behind them
+    const int rc = dalloc(&p->res_slots, nw + (sizeof(Fp64DevState) + 7) / 8);
+    if (rc) {
+        p->f64_planned = false;
+        return rc;
+    }
+    CU(cudaMemsetAsync(p->res_slots, 0, nw * sizeof *p->res_slots, p->stream));
+    p->st64 = reinterpret_cast<Fp64DevState *>(p->res_slots + nw);
+    p->st64_h = reinterpret_cast<Fp64DevState *>(p->red_out_h + 8);
+    p->f64_plan = plan;
+    return PASC_OK;
+}
 
 // n iterations while the solve runs (first: with the evaluation of the start point before them).
 // *refused: the device does not take the cooperative launch, and nothing was done.
@@ -823,6 +835,7 @@ static int fp64_fused_start(pasc_gb300_problem *p, long sweeps, bool *refused)
 // the path allows
 static int fp64_start(pasc_gb300_problem *p, long sweeps)
 {
+    CHK(fp64_prepare(p));
     if (fp64_fused(p)) {
         bool refused = false;
         CHK(fp64_fused_start(p, sweeps, &refused));

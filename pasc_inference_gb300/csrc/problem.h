@@ -54,6 +54,7 @@ struct pasc_gb300_problem {
     // fp64 iterations in one cooperative launch (kernels_fp64.cu); 0 blocks: one kernel per operation
     pasc::Fp64DevState *st64 = nullptr, *st64_h = nullptr;  // behind res_slots, red_out_h
     pasc::Fp64Plan f64_plan{};
+    bool f64_planned = false;
 
     // mixed path
     float *data32 = nullptr, *theta32 = nullptr;  // data32 points past the front pad
