@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "launch_rules.h"
 
 namespace pasc {
 
@@ -99,6 +100,7 @@ __global__ void fem_prolongate_kernel(const TIn *g2, TOut *g1, long T1, long T2,
 }
 
 // ---- FEM-SUM of the mixed path ----
+// (Signals that fem_sum_indexable accepts.)
 // lo[j]: the first fine timestep of coarse timestep j (lo[T2] = T1), computed once when the
 // reduction is set up: the FP64 rounding of the reference's expressions costs as much as the sums.
 // The fine field is read, and the prolongated one written, in consecutive order.  Sums: gamma, an
@@ -109,7 +111,7 @@ __global__ void fem_prolongate_kernel(const TIn *g2, TOut *g1, long T1, long T2,
 // values themselves; the result is rounded to FP32 either way.  (One thread per coarse entry,
 // summing in FP64 with a stride of K: 95 us for both reductions at T = 2e6, K = 3, T2 = T/10; here
 // 24 and 12, and the copy back 15.)
-constexpr int FEM_NT = 256;
+constexpr int FEM_NT = (int)FEM_SUM_THREADS;
 
 __global__ void __launch_bounds__(FEM_NT) fem_bounds_kernel(int *lo, long T2, double diff)
 {

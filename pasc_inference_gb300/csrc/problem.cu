@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "problem.h"
+#include "launch_rules.h"
 
 using namespace pasc;
 
@@ -400,7 +401,7 @@ static int fem_update_b_async(pasc_gb300_problem *p, int *launches)
         CU((launch_fem_reduce<double, double>(nullptr, p->data64, p->theta64, q->b, T, T2, K, type, q->coeffB, s)));
         CU((launch_fem_reduce<double, double>(p->x, nullptr, nullptr, q->x, T, T2, K, type, 1.0, s)));
     } else {
-        const bool sum = p->fem_lo != nullptr;  // FEM-SUM
+        const bool sum = p->fem_lo != nullptr;  // FEM-SUM within fem_sum_indexable
         if (p->xdim > 1) {
             // the full b = bscale ||X_t - theta_k||^2 (FP32), then its reduction rescaled
             CHK(mc_residual_async(p, launches));
@@ -1767,7 +1768,7 @@ int pasc_gb300_set_fem(pasc_gb300_problem *p, double fem_reduce, int fem_type)
         g = (long)sweep_tma_blocks_per_sm(p->K, true, true) * q->sms;
         q->grid_sweep_init[1] = (int)(g < nt_tma ? (g < 1 ? 1 : g) : nt_tma);
     }
-    if (p->precision == PASC_PREC_MIXED && fem_type == 0) {
+    if (p->precision == PASC_PREC_MIXED && fem_type == 0 && fem_sum_indexable(p->T, T2, p->K)) {
         const int rc = dalloc(&p->fem_lo, (size_t)T2 + 1);
         if (rc || launch_fem_bounds(p->fem_lo, p->T, T2, p->stream) != cudaSuccess) {
             free_all(q);
