@@ -24,6 +24,7 @@
 // of sweeps.  d'Ad is accumulated in the difference form 2*coeff*sum (d_{t+1}-d_t)^2, equal
 // to d'(A d) for the FEM-H1 matrix but free of the cancellation the dot form has in FP32.
 #include "common.cuh"
+#include "f3.cuh"
 #include "project.cuh"
 #include "internal.h"
 #include "sweep_common.cuh"
@@ -298,18 +299,25 @@ cudaError_t launch_sweep(int K, bool init, int grid, const SweepArgs &a, cudaStr
 // ---------------------------------------------------------------------------------------
 constexpr int THETA_NT = 256;
 
-// Per-thread sums compensated in FP32, block and grid sums float-float: with FP64 ones the four blocks
-// of an SM queued 120 FP64 warp instructions per warp at its slow FP64 pipe.  The loads of several
-// timesteps are issued together.  T = 2e6, K = 3: 30 us before, 17 now; T = 50 001, K = 4: 23, 11.
+// Per-thread sums compensated in FP32; warp sums in three FP32 terms (f3.cuh), which hold more than
+// FP64 does, block and grid sums in FP64.  With FP64 warp sums over every thread's pairs the four
+// blocks of an SM queued 120 FP64 warp instructions per warp at its slow FP64 pipe.  A warp with sums
+// near the end of the FP32 range (or not finite) takes FP64 for them.  The loads of several timesteps
+// are issued together.  us per update, FP64 sums in every thread / float-float ones / here: T = 2e6, K = 3
+// 30.8 / 17.0 / 16.5, K = 8 91 / 47.6 / 30.8; T = 50 001, K = 4 22.6 / 11.3 / 9.8.
 template <int K, bool TP = false>
 __global__ void __launch_bounds__(THETA_NT) theta_kernel(ThetaArgs a)
 {
     constexpr int NQ = TP ? 3 * K : 2 * K, U = K <= 3 ? 4 : (K <= 5 ? 2 : 1);
-    __shared__ float2 s_red[NQ * (THETA_NT / 32)];
+    constexpr int NW = THETA_NT / 32, GT = THETA_NT / NQ * NQ;
+    __shared__ float s_f3[NQ * NW][3];
+    __shared__ double s_red[THETA_NT];  // sums of the warps (NQ * NW), then of the grid's threads
+    __shared__ bool s_wide[NW];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float *gam = a.cur ? a.xb1 : a.xb0;
     KahanF sx[K], sg[K], sa[TP ? K : 1];
     const long stride = (long)gridDim.x * THETA_NT;
-    for (long t0 = (long)blockIdx.x * THETA_NT + threadIdx.x; t0 < a.T; t0 += U * stride) {
+    for (long t0 = (long)blockIdx.x * THETA_NT + tid; t0 < a.T; t0 += U * stride) {
         float x[U], g[U][K];
 #pragma unroll
         for (int u = 0; u < U; u++) {
@@ -335,35 +343,65 @@ __global__ void __launch_bounds__(THETA_NT) theta_kernel(ThetaArgs a)
             }
         }
     }
-    FF v[NQ];
+    F3 v[NQ];
+    bool narrow = true;  // a warp's 32 values stay in the FP32 range
 #pragma unroll
     for (int k = 0; k < K; k++) {
-        v[k] = FF{sx[k].s, sx[k].c};
-        v[K + k] = FF{sg[k].s, sg[k].c};
-        if (TP) v[(TP ? 2 * K : 0) + k] = FF{sa[TP ? k : 0].s, sa[TP ? k : 0].c};
+        v[k] = F3{sx[k].s, sx[k].c, 0.f};
+        v[K + k] = F3{sg[k].s, sg[k].c, 0.f};
+        if (TP) v[(TP ? 2 * K : 0) + k] = F3{sa[TP ? k : 0].s, sa[TP ? k : 0].c, 0.f};
     }
-    block_sum_ff<NQ>(v, s_red);
-    float2 *partials = reinterpret_cast<float2 *>(a.partials);
-    if (threadIdx.x == 0) {
 #pragma unroll
-        for (int q = 0; q < NQ; q++) partials[blockIdx.x * NQ + q] = make_float2(v[q].hi, v[q].lo);
-    }
-    if (!last_block_done(&a.st->counter2)) return;
-    FF u[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) u[q] = FF{0.f, 0.f};
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += THETA_NT) {
+    for (int q = 0; q < NQ; q++) narrow &= fabsf(v[q].a) < 0x1p122f && fabsf(v[q].b) < 0x1p122f;  // (false for NaN)
+    if (__all_sync(0xffffffffu, narrow)) {
+        f3_warp_sum<NQ>(v, lane);
+        const int q = f3_lane_value<NQ>(lane);
+        if (q >= 0) {
+            s_f3[q * NW + warp][0] = v[0].a;
+            s_f3[q * NW + warp][1] = v[0].b;
+            s_f3[q * NW + warp][2] = v[0].c;
+        }
+        if (lane == 0) s_wide[warp] = false;
+    } else {
 #pragma unroll
         for (int q = 0; q < NQ; q++) {
-            const float2 p = __ldcg(partials + b * NQ + q);
-            u[q] = ff_acc(u[q], FF{p.x, p.y});
+            double d[1] = {(double)v[q].a + (double)v[q].b};
+            warp_sum<1>(d);
+            if (lane == 0) s_red[q * NW + warp] = d[0];
         }
+        if (lane == 0) s_wide[warp] = true;
     }
-    block_sum_ff<NQ>(u, s_red);
-    if (threadIdx.x == 0) {
-        double w[NQ];
+    __syncthreads();
+    // eight neighbouring lanes per value, one for each warp's sum
+    static_assert(NW == 8 && NQ * NW <= THETA_NT, "a value of a warp per thread");
+    if (warp * 32 < NQ * NW) {
+        double d = 0.0;
+        if (tid < NQ * NW) d = s_wide[tid & 7] ? s_red[tid] : f3_value(F3{s_f3[tid][0], s_f3[tid][1], s_f3[tid][2]});
 #pragma unroll
-        for (int q = 0; q < NQ; q++) w[q] = ff_value(u[q]);
+        for (int m = 4; m >= 1; m >>= 1) d += __shfl_xor_sync(0xffffffffu, d, m);
+        if (tid < NQ * NW && (tid & 7) == 0) a.partials[blockIdx.x * NQ + (tid >> 3)] = d;
+    }
+    if (!last_block_done(&a.st->counter2)) return;
+    // over the blocks: thread i takes value i % NQ of every (GT / NQ)-th block, then a warp per value
+    {
+        double d = 0.0;
+        const int n = (int)gridDim.x * NQ;
+        if (tid < GT) {
+#pragma unroll 4
+            for (int i = tid; i < n; i += GT) d += __ldcg(a.partials + i);
+        }
+        s_red[tid] = d;
+    }
+    __syncthreads();
+    __shared__ double w[NQ];
+    for (int q = warp; q < NQ; q += NW) {
+        double d[1] = {0.0};
+        for (int j = lane; j < GT / NQ; j += 32) d[0] += s_red[j * NQ + q];
+        warp_sum<1>(d);
+        if (lane == 0) w[q] = d[0];
+    }
+    __syncthreads();
+    if (tid == 0) {
         a.st->counter2 = 0;
 #pragma unroll
         for (int k = 0; k < K; k++) {
