@@ -16,6 +16,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "f3.cuh"
 #include "internal.h"
 #include "launch_rules.h"
 
@@ -103,9 +104,9 @@ __global__ void fem_prolongate_kernel(const TIn *g2, TOut *g1, long T1, long T2,
 // (Signals that fem_sum_indexable accepts.)
 // lo[j]: the first fine timestep of coarse timestep j (lo[T2] = T1), computed once when the
 // reduction is set up: the FP64 rounding of the reference's expressions costs as much as the sums.
-// The fine field is read, and the prolongated one written, in consecutive order.  Sums: gamma, an
-// FP32 field, float-float; the residual in FP64 with three instead of 3K operations per fine
-// timestep,
+// The fine field is read, and the prolongated one written, in consecutive order.  Sums: an FP32
+// field in three FP32 terms (f3.cuh), which hold more than FP64 does, with FP64 where they leave the
+// FP32 range; the residual in FP64 with three instead of 3K operations per fine timestep,
 //     sum (x_t - theta_k)^2 = S2 - 2 e S1 + n e^2,   S1 = sum (x_t - c), S2 = sum (x_t - c)^2, e = theta_k - c
 // with c the block's first value, so that the cancellation is bounded by the spread of the
 // values themselves; the result is rounded to FP32 either way.  (One thread per coarse entry,
@@ -127,10 +128,15 @@ __global__ void __launch_bounds__(FEM_NT) fem_sum_field_kernel(const float *__re
     const unsigned int j = e / (unsigned int)K;
     const int k = (int)(e - j * K);
     const int hi = lo[j + 1];
-    FF s{0.f, 0.f};
-#pragma unroll 4
-    for (int i = lo[j]; i < hi; i++) s = ff_acc(s, ff_make(__ldg(g1 + (long)i * K + k)));
-    g2[e] = scale == 1.0 ? s.hi + s.lo : (float)__dmul_rn(ff_value(s), scale);
+    F3 s{0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int i = lo[j]; i < hi; i++) s = f3_add(s, __ldg(g1 + (long)i * K + k));
+    double sum = f3_value(s);
+    if (!isfinite(s.a)) {  // beyond the FP32 range, or a value that is not finite
+        sum = 0.0;
+        for (int i = lo[j]; i < hi; i++) sum = __dadd_rn(sum, (double)__ldg(g1 + (long)i * K + k));
+    }
+    g2[e] = (float)__dmul_rn(sum, scale);
 }
 
 template <int K>
