@@ -108,8 +108,11 @@ __global__ void fem_prolongate_kernel(const TIn *g2, TOut *g1, long T1, long T2,
 // field in three FP32 terms (f3.cuh), which hold more than FP64 does, with FP64 where they leave the
 // FP32 range; the residual in FP64 with three instead of 3K operations per fine timestep,
 //     sum (x_t - theta_k)^2 = S2 - 2 e S1 + n e^2,   S1 = sum (x_t - c), S2 = sum (x_t - c)^2, e = theta_k - c
-// with c the block's first value, so that the cancellation is bounded by the spread of the
-// values themselves; the result is rounded to FP32 either way.  (One thread per coarse entry,
+// with c the block's first value.  c is one of the summands, so S2 is at most 2 + 2n times the sum:
+// where the first value lies far from all others that is n digits' worth of cancellation, and
+// infinities give inf - inf.  Where the sum is below 2^-8 of S2 (c some 16 standard deviations off) or not a
+// number it is therefore taken term by term; elsewhere at most 11 of FP64's 53 bits are lost of a sum that
+// is stored in 24.  (One thread per coarse entry,
 // summing in FP64 with a stride of K: 95 us for both reductions at T = 2e6, K = 3, T2 = T/10; here
 // 24 and 12, and the copy back 15.)
 constexpr int FEM_NT = (int)FEM_SUM_THREADS;
@@ -159,7 +162,15 @@ __global__ void __launch_bounds__(FEM_NT) fem_sum_residual_kernel(const double *
 #pragma unroll
     for (int k = 0; k < K; k++) {
         const double d = theta[k] - c;
-        g2[(long)j * K + k] = (float)(fma(d, fma(n, d, u2), v) * scale);
+        double sum = fma(d, fma(n, d, u2), v);
+        if (!(sum >= 0x1p-8 * v)) {  // (also where it is NaN)
+            sum = 0.0;
+            for (int i = a; i < b; i++) {
+                const double r = data[i] - theta[k];
+                sum = __dadd_rn(sum, __dmul_rn(r, r));
+            }
+        }
+        g2[(long)j * K + k] = (float)__dmul_rn(sum, scale);
     }
 }
 
