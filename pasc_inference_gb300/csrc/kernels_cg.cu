@@ -7,17 +7,21 @@
 // alone, in the shared memory of the blocks, and an iteration (r and p to q = P A p and p'q; then d,
 // r and r'r) moves nothing through HBM.  Block b owns C consecutive entries of the list, thread i
 // M of them; rows are padded to an odd stride.  A neighbour in time that is not active has p = 0.
-// The two sums of an iteration are float-float and travel as tagged words (grid_words.cuh)
-// together with r at the block's two ends, from which the neighbours bring their copies of p forward
-// themselves.  Measured at T = 1e6, K = 3, 280 000 active timesteps: 26 us per iteration with one kernel
-// per half iteration over all timesteps, 6.9 here; 3.2 on three blocks.  What bounds it: the two
-// exchanges, 1.5 to 1.8 us each between the two dies.
+// The two sums of an iteration are FP64 (three FP32 terms up to a warp, f3.cuh) and travel as tagged
+// words (grid_words.cuh) together with r at the block's two ends, from which the neighbours bring their
+// copies of p forward themselves.  Warp 0 adds the blocks' sums and forms alpha and beta.  Measured at
+// T = 1e6, K = 3, 280 000 active timesteps: 26 us per iteration with one kernel per half iteration over all
+// timesteps, 6.9 here; 4.5 on eleven blocks, about 4 on one.  What bounds it: the two exchanges, 1.5 to 1.8 us each
+// between the two dies, and on few blocks warp 0's chain of FP64 operations (float-float sums and
+// quotients in every thread, with fewer bits, took 0.9 to 1.3 us less there, and up to 1.1 us more where many
+// entries share a block: T = 3e5, K = 8 7.1 against 5.9 ms an adjoint).
 //
 // The scalars follow adjoint.cu: alpha = r'r / p'q, beta the ratio of successive r'r, until r'r has
 // dropped by ADJ_INNER_TOL^2, maxit, or a breakdown (p'q <= 0).
 #include <algorithm>
 
 #include "common.cuh"
+#include "f3.cuh"
 #include "grid_words.cuh"
 #include "internal.h"
 #include "adjoint.h"
@@ -25,7 +29,7 @@
 namespace pasc {
 
 constexpr int CG_NT = 512;
-constexpr int CG_WORDS = 4 + 2 * KMAX_FUSED;  // a block's words: two sums (float-float), r at its two ends
+constexpr int CG_WORDS = 4 + 2 * KMAX_FUSED;  // a block's words: two sums (FP64), r at its two ends
 
 // entry flags above the mask's bits
 constexpr unsigned int CG_LEFT = 1u << 8, CG_RIGHT = 1u << 9;    // the timestep has one before / after it
@@ -34,66 +38,76 @@ constexpr unsigned int CG_LACT = 1u << 10, CG_RACT = 1u << 11;  // which is the 
 template <int K>
 struct CgSmem {
     float hr[2][K], hp[2][K];  // r, p of the entries before and after the block
-    float2 red[CG_NT / 32], red2[CG_NT / 32];
+    float red[CG_NT / 32][3];  // the warps' sums
+    // of the whole grid, from warp 0
+    float alpha, beta;
+    int status, it;
+    int gave_up;               // a wait gave up
 };
 
-__device__ __forceinline__ FF warp_sum_acc(FF r)
+// sum over lanes 0 .. n - 1 (the others hold 0), in lane 0
+__device__ __forceinline__ double warp_sum_of(double v, int n)
 {
+    for (int m = n > 16 ? 16 : (n > 8 ? 8 : (n > 4 ? 4 : (n > 2 ? 2 : 1))); m >= 1; m >>= 1)
+        v += __shfl_xor_sync(0xffffffffu, v, m);
+    return v;
+}
+
+// (float)(a / b).  A quotient of FP32 numbers and one correction from its FP64 remainder: off by 2^-46
+// before it is rounded to FP32.  (An FP64 division in its place: 0.2 to 0.4 us
+// more per iteration.)
+__device__ __forceinline__ float cg_quotient(double a, double b)
+{
+    const float fa = (float)a, fb = (float)b;
+    if (!(fabsf(fa) > 0x1p-60f && fabsf(fa) < 0x1p60f && fabsf(fb) > 0x1p-60f && fabsf(fb) < 0x1p60f)) return (float)(a / b);
+    const float q = fa / fb;
+    return q + (float)fma(-(double)q, b, a) / fb;
+}
+
+// A warp's share of a grid-wide sum: three FP32 terms within the warp (f3.cuh), FP64 beyond.
+__device__ __forceinline__ void cg_warp_sum(F3 v, float (*red)[3])
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) r = ff_acc(r, ff_shfl_xor(r, m));
-    return r;
+    for (int m = 16; m >= 1; m >>= 1) v = f3_add(v, f3_shfl_xor(v, m));
+    if (lane == 0) {
+        red[warp][0] = v.a;
+        red[warp][1] = v.b;
+        red[warp][2] = v.c;
+    }
 }
 
-// a / b rounded to FP32 from float-float operands (b.hi != 0): the quotient of the high parts and one
-// correction
-__device__ __forceinline__ float ff_quotient(FF a, FF b)
+// Warp 0: the sum over the block's warps, published, and the sum over all blocks, in lane 0.
+// slots: the blocks' words (CG_WORDS apart), which: the sum's place among them.  ok turns false
+// where a wait gave up.
+__device__ __forceinline__ double cg_grid_sum(const float (*red)[3], unsigned long long *slots, int which,
+                                              unsigned int tag, bool &ok)
 {
-    const float q = a.hi / b.hi;
-    const float rem = __fadd_rn(__fadd_rn(fmaf(-q, b.hi, a.hi), a.lo), -__fmul_rn(q, b.lo));
-    return __fadd_rn(q, rem / b.hi);
-}
-
-// Sum over all blocks, in every thread.  word: the block's slot of this exchange (of `slots`,
-// CG_WORDS apart).  ok turns false where a wait gave up.
-__device__ __forceinline__ FF cg_grid_sum(FF v, float2 *red, float2 *red2, unsigned long long *slots, int which,
-                                          unsigned int tag, bool &ok)
-{
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5, nb = gridDim.x;
-    v = warp_sum_acc(v);
-    if (lane == 0) red[warp] = make_float2(v.hi, v.lo);
-    __syncthreads();
-    if (nb == 1) {
-        FF t{0.f, 0.f};
-        for (int q = 0; q < nw; q++) t = ff_acc(t, FF{red[q].x, red[q].y});
-        __syncthreads();
-        return t;
-    }
-    if (warp == 0) {
-        const float2 p = lane < nw ? red[lane] : make_float2(0.f, 0.f);
-        const FF t = warp_sum_acc(FF{p.x, p.y});
-        if (lane == 0)
-            word_store2(slots + (size_t)blockIdx.x * CG_WORDS + 2 * which, word_of(t.hi, tag), word_of(t.lo, tag));
-    }
-    const int polling = (nb + 31) / 32;  // warps that poll, one block per lane
-    if (warp < polling) {
-        FF u{0.f, 0.f};
-        if (tid < nb) {
-            unsigned long long hi = 0, lo = 0;
-            bool have = false;
-            for (unsigned int it = 0; it < WORD_WAIT_LIMIT && !have; it++) {
-                word_load2(slots + (size_t)tid * CG_WORDS + 2 * which, hi, lo);
-                have = word_valid(hi, tag) && word_valid(lo, tag);
+    constexpr int POLL = 5;  // words a lane has in flight
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, nb = gridDim.x;
+    const double own = warp_sum_of(lane < nw ? f3_value(F3{red[lane][0], red[lane][1], red[lane][2]}) : 0.0, nw);
+    if (nb == 1) return own;
+    if (lane == 0) word_store_double(slots + (size_t)blockIdx.x * CG_WORDS + 2 * which, own, tag);
+    double sum = 0.0;
+    for (int b0 = lane; b0 < nb; b0 += 32 * POLL) {
+        unsigned long long hi[POLL], lo[POLL];
+        bool have = false;
+        for (unsigned int it = 0; it < WORD_WAIT_LIMIT && !have; it++) {
+            have = true;
+#pragma unroll
+            for (int q = 0; q < POLL; q++) {
+                const int b = b0 + 32 * q;
+                if (b < nb) word_load2(slots + (size_t)b * CG_WORDS + 2 * which, hi[q], lo[q]);
+                else hi[q] = lo[q] = word_of(0u, tag);
             }
-            ok &= have;
-            u = FF{word_float(hi), word_float(lo)};
+#pragma unroll
+            for (int q = 0; q < POLL; q++) have &= word_valid(hi[q], tag) && word_valid(lo[q], tag);
         }
-        u = warp_sum_acc(u);
-        if (lane == 0) red2[warp] = make_float2(u.hi, u.lo);
+        ok &= have;
+#pragma unroll
+        for (int q = 0; q < POLL; q++) sum += __hiloint2double((int)(unsigned int)hi[q], (int)(unsigned int)lo[q]);
     }
-    ok = __syncthreads_and(ok);
-    FF t{0.f, 0.f};
-    for (int q = 0; q < polling; q++) t = ff_acc(t, FF{red2[q].x, red2[q].y});
-    return t;
+    return warp_sum_of(sum, nb);
 }
 
 template <int K>
@@ -134,12 +148,12 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
     float *r = rs + tid * S, *p = ps + tid * S, *q = qs + tid * S, *d = ds + tid * S;
     const unsigned short *fl = fs + tid * M;
     const float coeff = a.coeff;
-    const double rr_in = a.st->rr, stop = ADJ_INNER_TOL * ADJ_INNER_TOL * a.st->rr_in0;
-    FF rr{(float)rr_in, (float)(rr_in - (double)(float)rr_in)};
-    const FF lim{(float)stop, (float)(stop - (double)(float)stop)};
+    double rr = a.st->rr;  // (thread 0)
+    const double stop = ADJ_INNER_TOL * ADJ_INNER_TOL * a.st->rr_in0;
     const int maxit = a.st->maxit;
     int it = a.st->it, status = ADJ_RUNNING;
     float beta = a.resume ? (float)a.st->beta : 0.f;
+    if (tid == 0) sm.gave_up = 0;
     bool ok = true;
     __syncthreads();
 
@@ -159,7 +173,7 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
             }
         }
         __syncthreads();  // the neighbours' rows were read
-        FF pq{0.f, 0.f};
+        F3 pq{0.f, 0.f, 0.f};
         if (m > 0) {
             if (tid == 0) {
 #pragma unroll
@@ -194,17 +208,27 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
                     pl[k] = pc[k];
                     pc[k] = pn[k];
                 }
-                pq = ff_acc(pq, ff_make(part));
+                pq = f3_add(pq, part);
             }
         }
-        pq = cg_grid_sum(pq, sm.red, sm.red2, slots, 0, tag, ok);
-        if (!ok) break;
-        if (!(pq.hi > 0.f) || !isfinite(pq.hi)) {
-            status = ADJ_BREAKDOWN;
-            break;
+        cg_warp_sum(pq, sm.red);
+        __syncthreads();
+        if (tid < 32) {
+            const double sum = cg_grid_sum(sm.red, slots, 0, tag, ok);
+            if (!__all_sync(0xffffffffu, ok)) sm.gave_up = 1;
+            if (tid == 0) {
+                const bool fine = sum > 0.0 && isfinite(sum);
+                sm.alpha = fine ? cg_quotient(rr, sum) : 0.f;
+                sm.status = fine ? ADJ_RUNNING : ADJ_BREAKDOWN;
+            }
         }
-        const float alpha = ff_quotient(rr, pq);
-        FF rn{0.f, 0.f};
+        __syncthreads();
+        ok = sm.gave_up == 0;
+        if (!ok) break;
+        status = sm.status;
+        if (status != ADJ_RUNNING) break;
+        const float alpha = sm.alpha;
+        F3 rn{0.f, 0.f, 0.f};
 #pragma unroll 1
         for (int j = 0; j < m; j++) {
             float part = 0.f;
@@ -222,7 +246,7 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
                     if (last && j == m - 1) word_store(own + K + k, word_of(v, tag));
                 }
             }
-            rn = ff_acc(rn, ff_make(part));
+            rn = f3_add(rn, part);
         }
         // (the neighbours' r at this block's ends are awaited with the sum)
         if (nb > 1 && tid >= nt - 2 * K) {
@@ -235,23 +259,29 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
                     v = word_load(w);
                     have = word_valid(v, tag);
                 }
-                ok &= have;
+                if (!have) sm.gave_up = 1;
                 sm.hr[e][k] = word_float(v);
             }
         }
-        rn = cg_grid_sum(rn, sm.red, sm.red2, slots, 1, tag, ok);
+        cg_warp_sum(rn, sm.red);
+        __syncthreads();
+        if (tid < 32) {
+            const double sum = cg_grid_sum(sm.red, slots, 1, tag, ok);
+            if (!__all_sync(0xffffffffu, ok)) sm.gave_up = 1;
+            if (tid == 0) {
+                sm.beta = cg_quotient(sum, rr);
+                sm.it = it + 1;
+                sm.status = !isfinite(sum) ? ADJ_BREAKDOWN : (sum <= stop || it + 1 >= maxit ? ADJ_INNER_DONE : ADJ_RUNNING);
+            }
+            rr = sum;
+        }
+        __syncthreads();
+        ok = sm.gave_up == 0;
         if (!ok) break;
-        beta = ff_quotient(rn, rr);
-        rr = rn;
-        it++;
-        if (!isfinite(rr.hi)) {
-            status = ADJ_BREAKDOWN;
-            break;
-        }
-        if ((rr.hi - lim.hi) + (rr.lo - lim.lo) <= 0.f || it >= maxit) {
-            status = ADJ_INNER_DONE;
-            break;
-        }
+        status = sm.status;
+        beta = sm.beta;
+        it = sm.it;
+        if (status != ADJ_RUNNING) break;
     }
     if (!ok) {
         if (tid == 0) {
@@ -274,7 +304,7 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
         }
     }
     if (blockIdx.x == 0 && tid == 0) {
-        a.st->rr = (double)rr.hi + (double)rr.lo;
+        a.st->rr = rr;
         a.st->beta = beta;
         a.st->it = it;
         a.st->status = status;
@@ -394,8 +424,7 @@ bool cg_plan(int K, long n, int sms, CgPlan *p)
     p->blocks = (int)((n + C - 1) / C);
     p->C = (int)C;
     p->M = (int)M;
-    // (at least the warps that poll the blocks' words)
-    p->threads = (int)std::max((rows + 31) / 32, (long)(p->blocks + 31) / 32) * 32;
+    p->threads = (int)((rows + 31) / 32) * 32;
     p->smem = smem;
     // (the same limit for every handle: all a block can have)
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room) != cudaSuccess ||
