@@ -8,7 +8,7 @@
 // g^{c+1}, d_{c+2} and its sums from the neighbours' x^{c+1}, which it recomputes in a halo (read x, d
 // and data, write x and d: (16 K + 4) bytes per pixel).  Recomputing d_{c+1} from x^c instead of
 // storing it moves (8 K + 4) bytes but takes a second projection and stencil per pixel and a
-// halo of 3; it was issue-bound at 388 instructions per owned pixel (IMAGE_NOTE).
+// halo of 3; it was issue-bound at 388 instructions per owned pixel (K = 3).
 //
 // Each warp takes a strip tile: 32 columns (one per lane; 29 owned, one more on the left and two on
 // the right) by th + 3 rows (the middle th owned), walked top to bottom with everything in registers:
@@ -17,7 +17,7 @@
 //              d'd, g'd, the pair with the right neighbour, and the store of x^{c+1} and d_{c+2}; the
 //              pair with the row above belongs to that row.
 // Left and right neighbours come from the adjacent lanes (shuffles), up and down from the
-// three-row windows; there is no shared memory and no block barrier in the sweep.  Strip tiles
+// three-row windows; there is no block barrier in the sweep.  Strip tiles
 // away from the image border run without range checks.
 // Pixels outside the image hold zeros and are no one's neighbours.  The last block applies the
 // step-length / GLL / stop logic of the 1-D sweeps (sweep_common.cuh).
@@ -31,9 +31,89 @@
 
 namespace pasc {
 
-constexpr int IMG_NT = 256;                  // 8 warps, each on its own strip tile
 constexpr int IMG_TW = 29;                   // owned columns per warp (one lane per column)
-constexpr int IMG_PF = 3;                    // rows in flight per warp (a multiple of the 3-row windows)
+
+// Threads of a block (each warp on its own strip tile), blocks per SM its registers leave room for, and
+// rows a warp has in flight.
+// A pixel's K values lie side by side, so a store of one value per lane touches a sector per lane: 2 K
+// such stores per pixel were what bounded large images with many clusters, and the 160 to 200 registers
+// of K >= 5 left one block of 8 warps per SM.  Even K >= 6 moves 8 or 16
+// bytes at a time, K = 5 and 7 (odd: no wider alignment) write through shared memory.  us per sweep,
+// recomputed direction / stored one, a value at a time / here: K = 5, 1920 x 1080 112 / 70 / 43, 4096 x 4096
+// 474 / 398 / 274; K = 6 116 / 100 / 46, 497 / 705 / 291; K = 7 148 / 131 / 69, 597 / 978 / 417; K = 8 196 / 162 /
+// 57, 935 / 1180 / 386.  Shapes tried at 4096 x 4096: K = 7 4 blocks, 2 rows 459, 3 blocks, 3 rows 417; K = 8 4
+// blocks, 2 rows 500, 3 blocks, 3 rows 406, 4 blocks, 1 row 386; K = 6 5 blocks, 2 rows 384.  K = 3, two blocks of
+// 256: 28.4 at 1920 x 1080; the compiler's own choice 31.2, three blocks 39.0.
+template <int K>
+struct ImgShape {
+    static constexpr int NT = K <= 4 ? 256 : 128, BLOCKS = K <= 4 ? 2 : (K == 7 ? 3 : 4);
+    static constexpr int PF = K <= 4 || K == 7 ? 3 : (K == 8 ? 1 : 2);
+    static constexpr int VEC = K == 8 ? 4 : (K == 6 ? 2 : 1);  // values per load and store
+    static constexpr bool STAGED = K == 5 || K == 7;           // stores through shared memory
+};
+
+template <int V>
+struct ImgVec;
+template <>
+struct ImgVec<1> {
+    using type = float;
+};
+template <>
+struct ImgVec<2> {
+    using type = float2;
+};
+template <>
+struct ImgVec<4> {
+    using type = float4;
+};
+
+// the K values of one pixel (rows of K * 4 bytes: aligned to 4 VEC)
+template <int K>
+__device__ __forceinline__ void image_load_pixel(const float *__restrict__ p, bool in, float (&v)[K])
+{
+    constexpr int V = ImgShape<K>::VEC;
+    using T = typename ImgVec<V>::type;
+#pragma unroll
+    for (int k = 0; k < K; k += V) {
+        T t{};
+        if (in) t = __ldg(reinterpret_cast<const T *>(p + k));
+        const float *f = reinterpret_cast<const float *>(&t);
+#pragma unroll
+        for (int j = 0; j < V; j++) v[k + j] = f[j];
+    }
+}
+template <int K>
+__device__ __forceinline__ void image_store_pixel(float *p, const float (&v)[K])
+{
+    constexpr int V = ImgShape<K>::VEC;
+    using T = typename ImgVec<V>::type;
+#pragma unroll
+    for (int k = 0; k < K; k += V) {
+        T t{};
+        float *f = reinterpret_cast<float *>(&t);
+#pragma unroll
+        for (int j = 0; j < V; j++) f[j] = v[k + j];
+        *reinterpret_cast<T *>(p + k) = t;
+    }
+}
+
+// The owned pixels of a row, one per lane in v, written as consecutive values (whole warp; p: lane 0's
+// pixel, of which and of the two last lanes' nothing is written; cols: columns of the image from there
+// on; buf: 32 * K values of shared memory).
+template <int K>
+__device__ __forceinline__ void image_store_row(float *p, const float (&v)[K], int cols, float *buf)
+{
+    const int lane = threadIdx.x & 31, n = min(IMG_TW + 1, cols) * K;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < K; k++) buf[lane * K + k] = v[k];
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < K; m++) {
+        const int e = lane + 32 * m;
+        if (e >= K && e < n) p[e] = buf[e];
+    }
+}
 
 // x^c, d and data of staged row i of a strip tile (zeros outside the image)
 template <int K, bool INIT, bool EDGE>
@@ -44,17 +124,17 @@ __device__ __forceinline__ void image_load_row(const ImageSweepArgs &a, const fl
     const int gy = oy + i;
     const bool in = colin && (!EDGE || (unsigned)gy < (unsigned)H);
     const long pix = (long)gy * W + gx;
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        x[k] = in ? __ldg(xin + pix * K + k) : 0.f;
-        if (!INIT) d[k] = in ? __ldg(din + pix * K + k) : 0.f;
-    }
+    image_load_pixel<K>(xin + pix * K, in, x);
+    if (!INIT) image_load_pixel<K>(din + pix * K, in, d);
     v = in ? __ldg(a.data + pix) : 0.f;
 }
 
+template <int K>
 struct ImgSmem {
-    double red[4 * (IMG_NT / 32)];
+    static constexpr int WARPS = ImgShape<K>::NT / 32;
+    double red[4 * WARPS];
     SpgDevState snap;
+    float out[ImgShape<K>::STAGED ? WARPS * 32 * K : 1];
 };
 
 // sum over the in-image neighbours of (v_c - v_n); l, r from the neighbouring lanes, u, d from
@@ -78,9 +158,11 @@ template <int K, bool INIT, bool EDGE>
 __device__ __forceinline__ void image_strip(const ImageSweepArgs &a, const float *__restrict__ xin,
                                             const float *__restrict__ din, float *__restrict__ xout,
                                             float *__restrict__ dout, int ox, int oy, const float (&theta)[K],
-                                            float beta, float a1, float coeff, float bscale, KahanF &acc_f,
+                                            float beta, float a1, float coeff, float bscale, float *stage, KahanF &acc_f,
                                             FF &acc_dd, FF &acc_gd, FF &acc_dad)
 {
+    constexpr int IMG_PF = ImgShape<K>::PF;
+    constexpr bool STAGED = ImgShape<K>::STAGED;
     const int lane = threadIdx.x & 31;
     const int W = a.W, H = a.H, th = a.th, rows = th + 3;
     const int gx = ox + lane;
@@ -152,27 +234,33 @@ __device__ __forceinline__ void image_strip(const ImageSweepArgs &a, const float
                 if (r <= th) {
                     acc_f.add(fpart);
                     float dd = 0.f, gd = 0.f;
-                    const long pix = (long)gy * W + gx;
 #pragma unroll
                     for (int k = 0; k < K; k++) {
                         dd = fmaf(d1[k], d1[k], dd);
                         gd = fmaf(g1[k], d1[k], gd);
-                        xout[pix * K + k] = Y1[k];
-                        dout[pix * K + k] = d1[k];
+                    }
+                    if (!STAGED) {
+                        const long pix = (long)gy * W + gx;
+                        image_store_pixel<K>(xout + pix * K, Y1);
+                        image_store_pixel<K>(dout + pix * K, d1);
                     }
                     acc_dd = ff_acc(acc_dd, ff_make(dd));
                     acc_gd = ff_acc(acc_gd, ff_make(gd));
                 }
             }
+            if (STAGED && r <= th && (!EDGE || (unsigned)gy < (unsigned)H)) {  // uniform
+                const long first = (long)gy * W + ox;
+                image_store_row<K>(xout + first * K, Y1, W - ox, stage);
+                image_store_row<K>(dout + first * K, d1, W - ox, stage);
+            }
         }
     }
 }
 
-// (two blocks per SM: K = 3 at 1920 x 1080 28.4 us; the compiler's own choice 31.2, three blocks 39.0)
 template <int K, bool INIT>
-__global__ void __launch_bounds__(IMG_NT, K <= 4 ? 2 : 1) image_sweep_kernel(ImageSweepArgs a)
+__global__ void __launch_bounds__(ImgShape<K>::NT, ImgShape<K>::BLOCKS) image_sweep_kernel(ImageSweepArgs a)
 {
-    __shared__ ImgSmem sm;
+    __shared__ ImgSmem<K> sm;
     SpgDevState *st = a.st;
     if (st->status != PASC_SPG_RUNNING) return;  // uniform across the grid
     const int cur = st->cur;
@@ -186,7 +274,8 @@ __global__ void __launch_bounds__(IMG_NT, K <= 4 ? 2 : 1) image_sweep_kernel(Ima
     for (int k = 0; k < K; k++) theta[k] = a.theta[k];
     const int tiles_x = (W + IMG_TW - 1) / IMG_TW, tiles_y = (H + th - 1) / th;
     const int ntiles = tiles_x * tiles_y;
-    const int warps = IMG_NT / 32, warp = threadIdx.x >> 5;
+    const int warps = ImgShape<K>::NT / 32, warp = threadIdx.x >> 5;
+    float *stage = sm.out + (ImgShape<K>::STAGED ? warp * 32 * K : 0);
 
     // (the pixels' terms are added in float-float: the sums then hardly depend on th and the grid)
     KahanF acc_f;
@@ -195,11 +284,11 @@ __global__ void __launch_bounds__(IMG_NT, K <= 4 ? 2 : 1) image_sweep_kernel(Ima
         const int ty = tile / tiles_x, tx = tile - ty * tiles_x;
         const int ox = tx * IMG_TW - 1, oy = ty * th - 1;  // staged origin
         if (ox >= 0 && oy >= 0 && ox + 32 <= W && oy + th + 3 <= H)
-            image_strip<K, INIT, false>(a, xin, din, xout, dout, ox, oy, theta, beta, a1, coeff, bscale, acc_f, acc_dd,
-                                        acc_gd, acc_dad);
+            image_strip<K, INIT, false>(a, xin, din, xout, dout, ox, oy, theta, beta, a1, coeff, bscale, stage, acc_f,
+                                        acc_dd, acc_gd, acc_dad);
         else
-            image_strip<K, INIT, true>(a, xin, din, xout, dout, ox, oy, theta, beta, a1, coeff, bscale, acc_f, acc_dd,
-                                       acc_gd, acc_dad);
+            image_strip<K, INIT, true>(a, xin, din, xout, dout, ox, oy, theta, beta, a1, coeff, bscale, stage, acc_f,
+                                       acc_dd, acc_gd, acc_dad);
     }
 
     // d'A_hat d = sum over pairs of (d_p - d_n)^2; the finish step takes dAd = 2 coeff w[2]
@@ -217,15 +306,18 @@ template <int K, bool INIT>
 static int image_blocks_t()
 {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, image_sweep_kernel<K, INIT>, IMG_NT, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, image_sweep_kernel<K, INIT>, ImgShape<K>::NT, 0);
     return nb > 0 ? nb : 1;
 }
 
-// blocks per SM of the regular form
-static int image_blocks_per_sm(int K)
+// blocks per SM of the regular form, and warps of a block
+static int image_blocks_per_sm(int K, int *warps)
 {
     switch (K) {
-#define PASC_CASE(KK) case KK: return image_blocks_t<KK, false>();
+#define PASC_CASE(KK)                       \
+    case KK:                                \
+        *warps = ImgShape<KK>::NT / 32;     \
+        return image_blocks_t<KK, false>();
         PASC_CASE(1) PASC_CASE(2) PASC_CASE(3) PASC_CASE(4)
         PASC_CASE(5) PASC_CASE(6) PASC_CASE(7) PASC_CASE(8)
 #undef PASC_CASE
@@ -239,8 +331,10 @@ static int image_blocks_per_sm(int K)
 // 32.6, 24 (1.24) 36.4, 63 (0.5) 40.6; at 640 x 480: 6 13.5, 15 14.9, 63 35.
 void image_sweep_plan(int K, int W, int H, int sms, int *th, int *blocks)
 {
-    const int cols = (W + IMG_TW - 1) / IMG_TW, warps = IMG_NT / 32;
-    const long resident = std::max(1L, (long)image_blocks_per_sm(K) * sms * warps);
+    const int cols = (W + IMG_TW - 1) / IMG_TW;
+    int warps = 1;
+    const int per_sm = image_blocks_per_sm(K, &warps);
+    const long resident = std::max(1L, (long)per_sm * sms * warps);
     long best = LONG_MAX, tiles = 1;
     for (int t = 3; t <= 63; t += 3) {
         const long n = (long)cols * ((H + t - 1) / t), cost = (n + resident - 1) / resident * (t + 6);
@@ -258,8 +352,8 @@ cudaError_t launch_image_sweep(int K, bool init, int grid, const ImageSweepArgs 
     switch (K) {
 #define PASC_CASE(KK)                                                                                  \
     case KK:                                                                                           \
-        if (init) image_sweep_kernel<KK, true><<<grid, IMG_NT, 0, s>>>(a);                             \
-        else image_sweep_kernel<KK, false><<<grid, IMG_NT, 0, s>>>(a);                                 \
+        if (init) image_sweep_kernel<KK, true><<<grid, ImgShape<KK>::NT, 0, s>>>(a);                   \
+        else image_sweep_kernel<KK, false><<<grid, ImgShape<KK>::NT, 0, s>>>(a);                       \
         break;
         PASC_CASE(1) PASC_CASE(2) PASC_CASE(3) PASC_CASE(4)
         PASC_CASE(5) PASC_CASE(6) PASC_CASE(7) PASC_CASE(8)
