@@ -97,6 +97,7 @@ struct Fp64DevState {
     int fs_last, m, maxit, coeffmode;
     int stop_difff, stop_normgp, stop_normgp_normb, stop_Anormgp, stop_Anormgp_normb;
     int it, hessmult, status, sweeps, error;
+    int ahead;  // the status is that of the next direction, which is formed with the last step
 };
 
 struct Fp64Plan {

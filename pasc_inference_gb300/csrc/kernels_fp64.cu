@@ -155,6 +155,7 @@ __device__ __forceinline__ void f64_finish(Fp64DevState &h, F64Step &out, double
             h.dd = dd;
             h.dAd = dAd;
             h.gd = gd;
+            h.ahead = status != PASC_SPG_RUNNING;
         }
         h.status = status;
         out.beta = h.beta;

@@ -744,6 +744,7 @@ static int fp64_fused_run(pasc_gb300_problem *p, bool first, long n, bool *refus
     Fp64DevState *h = p->st64_h;
     // sweeps of one launch at most, about a tenth of a second: other work on the GPU gets its turn
     const long most = std::max(16L, std::min(4096L, 4000000000L / std::max(1L, p->N)));
+    const long target = r.it + n;
     long left = n + (first ? 1 : 0);
     bool begin = first;
     do {
@@ -784,6 +785,13 @@ static int fp64_fused_run(pasc_gb300_problem *p, bool first, long n, bool *refus
     r.it = h->it;
     r.hessmult = h->hessmult;
     r.status = h->status;
+    if (r.it == target && (r.status == PASC_SPG_RUNNING || h->ahead)) {
+        // the direction after the last iteration asked for is at hand already, but belongs to the
+        // next call: its product and what it says about the solve are reported there
+        r.hessmult -= 1;
+        r.pending = r.status == PASC_SPG_RUNNING ? 0 : r.status;
+        r.status = PASC_SPG_RUNNING;
+    }
     r.fx = h->fx;
     r.fx_old = h->fx_old;
     r.dd = h->dd_done;
@@ -890,7 +898,11 @@ static int fp64_iterate(pasc_gb300_problem *p, long n)
     double v[3];
     if (fp64_fused(p)) {
         n = std::min(n, (long)o->maxit - r.it);
-        if (r.status == PASC_SPG_RUNNING && n > 0) {
+        if (r.status == PASC_SPG_RUNNING && n > 0 && r.pending) {
+            r.status = r.pending;
+            r.pending = 0;
+            r.hessmult += 1;
+        } else if (r.status == PASC_SPG_RUNNING && n > 0) {
             bool refused = false;
             CU(cudaEventRecord(p->ev0, s));
             CHK(fp64_fused_run(p, false, n, &refused));

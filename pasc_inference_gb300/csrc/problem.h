@@ -24,6 +24,7 @@ struct SpgRun {
     double time_s = 0.0;
     float last_iterate_ms = 0.f;
     int last_iterate_launches = 0;
+    int pending = 0;     // FP64 in one launch: status of the direction formed ahead, for the next call
 };
 }  // namespace pasc
 
