@@ -212,7 +212,8 @@ int pasc_gb300_spgqp_solve(pasc_gb300_problem *p, const pasc_gb300_spgqp_opts *o
 int pasc_gb300_spgqp_start(pasc_gb300_problem *p, const pasc_gb300_spgqp_opts *o);
 int pasc_gb300_spgqp_iterate(pasc_gb300_problem *p, long n, int poll, pasc_gb300_spgqp_stats *st);
 /* Device time (CUDA events on the problem's stream) and kernel launches of the last
- * spgqp_iterate call. */
+ * spgqp_iterate call, or of the iterations of the last spgqp_solve (mixed path; a solve in one
+ * cooperative launch makes its start in that launch too). */
 int pasc_gb300_spgqp_last_iterate(pasc_gb300_problem *p, double *ms, int *launches);
 
 /* Sweep kernel of the mixed path (no reference counterpart: the reference has one SpMV and

@@ -62,7 +62,7 @@ struct pasc_gb300_problem {
     float *xb[2] = {nullptr, nullptr};            // past the front pad of xb_raw
     float *xb_raw[2] = {nullptr, nullptr}, *data32_raw = nullptr;
     pasc::SpgDevState *st = nullptr, *st_h = nullptr;  // st_h: three mirrors (the state, two polls in flight)
-    cudaEvent_t ev_poll[2] = {nullptr, nullptr};
+    cudaEvent_t ev_init = nullptr, ev_poll[2] = {nullptr, nullptr};  // end of the INIT sweep; polls
     bool start_in_flight = false;  // the INIT sweep was launched by a solve that iterates at once: not read back yet
     double *partials = nullptr;
     int cur = 0;
