@@ -1030,7 +1030,7 @@ static int adj_refine(pasc_gb300_problem *p, AdjDevState *h, int *launches)
                 a.resume = resume ? 1 : 0;
                 a.coeff = (float)p->coeffA;
                 const cudaError_t e = launch_cg(p->K, w->cg, a, s);
-                if (e == cudaErrorCooperativeLaunchTooLarge && !resume) {
+                if (cooperative_refused(e) && !resume) {
                     // the device does not take the launch (an SM partition, say): all timesteps, from
                     // the same residual
                     cudaGetLastError();

@@ -86,6 +86,13 @@ struct ResidentArgs {
     int sweeps;  // at most this many (the solve may end earlier)
 };
 
+// What a cooperative launch answers where the device does not take it, and nothing has run: the call
+// goes on with ordinary launches.
+inline bool cooperative_refused(cudaError_t e)
+{
+    return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported || e == cudaErrorNotPermitted;
+}
+
 // Device-resident state of one FP64 solve (kernels_fp64.cu).
 struct Fp64DevState {
     double alpha, beta;     // step length of the direction at hand, its line-search step

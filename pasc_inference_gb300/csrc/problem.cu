@@ -764,7 +764,7 @@ static int fp64_fused_run(pasc_gb300_problem *p, bool first, long n, bool *refus
         a.first = begin ? 1 : 0;
         a.sweeps = (int)std::min(left, most);
         const cudaError_t e = launch_fp64_iterations(p->K, p->f64_plan, a, s);
-        if (e == cudaErrorCooperativeLaunchTooLarge && begin) {
+        if (cooperative_refused(e) && begin) {
             cudaGetLastError();
             *refused = true;
             return PASC_OK;
@@ -845,8 +845,8 @@ static int fp64_fused_start(pasc_gb300_problem *p, long sweeps, bool *refused)
 static int fp64_start(pasc_gb300_problem *p, long sweeps)
 {
     CHK(fp64_prepare(p));
+    bool refused = false;
     if (fp64_fused(p)) {
-        bool refused = false;
         CHK(fp64_fused_start(p, sweeps, &refused));
         if (!refused) return PASC_OK;
         p->f64_plan.blocks = 0;  // from here on one kernel per operation
@@ -864,7 +864,7 @@ static int fp64_start(pasc_gb300_problem *p, long sweeps)
     CHK(read_red(p, 1, v));
     r.normb = sqrt(v[0]);             // :104
     r.alpha = r.o.alphainit;          // :108
-    CU(launch_project_f64(p->x, T, K, s));                   // :116
+    if (!refused) CU(launch_project_f64(p->x, T, K, s));     // :116 (else it is done)
     // :122-123; SPGQPSolverC (spgqpsolver_coeff.h:667-668) multiplies with coefficient 1 and
     // scales by eps afterwards: 1.0 * sum is exact, so eps * sum is the same value
     CU(apply_A_f64(p, p->x, p->g, s, p->coeffA));
@@ -1336,7 +1336,7 @@ static int resident_run(pasc_gb300_problem *p, bool init, long n)
         a.sweeps = (int)(left < RESIDENT_MAX_SWEEPS ? left : RESIDENT_MAX_SWEEPS);
         a.tag = p->res_tag;
         cudaError_t e = launch_resident(p->K, p->res_mode, p->res_plan, a, s);
-        if (e == cudaErrorCooperativeLaunchTooLarge && launches == 0) {
+        if (cooperative_refused(e) && launches == 0) {
             cudaGetLastError();
             p->res_refused = true;
             p->res_used = false;
