@@ -43,7 +43,8 @@ enum pasc_gb300_error {
     PASC_ERR_ALLOC = 3,     /* device or host allocation failed */
     PASC_ERR_STATE = 4,     /* call not valid in the handle's current state */
     PASC_ERR_NOTSUPP = 5,   /* configuration not supported by the library */
-    PASC_ERR_TIMEOUT = 6    /* a bounded device wait gave up */
+    PASC_ERR_TIMEOUT = 6    /* a bounded device wait gave up; gamma and the call's results are undefined
+                               then (the handle stays usable: set gamma again) */
 };
 
 /* Solve outcome reported in pasc_gb300_spgqp_stats.status. */

@@ -626,7 +626,9 @@ __global__ void __launch_bounds__(ResShape<K>::NT + RES_MGR, 1) spg_resident_ker
         if (mw == 0 && plain && sm.status == PASC_SPG_RUNNING) res_record<K>(sm, value, nbeta, nalpha, lane);
     }
     __syncthreads();
-    if (sm.status < 0) return;  // a wait gave up: the error word is set, gamma is left as it was
+    // a wait gave up: the error word is set.  (gamma is undefined then: blocks that had all they waited for
+    // in the last sweep write their rows.)
+    if (sm.status < 0) return;
     for (int tl = tid; tl < Cb; tl += nt) {
         const int i = tl / M, j = tl - i * M;
 #pragma unroll

@@ -1108,7 +1108,8 @@ static int ensure_chunk_graph(pasc_gb300_problem *p)
 static int check_device_error(pasc_gb300_problem *p)
 {
     if (p->st_h->error)
-        return fail(PASC_ERR_TIMEOUT, "spgqp: a bounded wait for a bulk copy gave up inside the sweep");
+        return fail(PASC_ERR_TIMEOUT, "spgqp: a bounded wait for %s gave up inside the sweep",
+                    p->res_used ? "another block" : "a bulk copy");
     return PASC_OK;
 }
 

@@ -3,6 +3,10 @@ ordinary launches.  The refusal is made on the host: the library's objects are l
 cudaLaunchCooperativeKernel replaced by a function that answers an error code (nothing is launched
 then), and a child process runs on that library.
 
+The same library with a cooperative launch one block short: the block before the missing one waits for
+edges that nobody writes.  The wait is bounded (a few seconds), the call reports it, and the handle solves
+again afterwards.  (Every index stays within the buffers, which hold the words of a block per SM.)
+
 Results against the same calls with the launches accepted: FP64 bit for bit (the paths keep one order of
 sums), mixed solves within the bounds of test_gpu_resident, gradients within those of test_gpu_cg."""
 import glob
@@ -19,13 +23,14 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SHIM = r"""
 #include <cuda_runtime.h>
 extern "C" {
-int coop_answer = 0;   // 0: the real launch; otherwise the error it answers
+int coop_answer = 0;   // 0: the real launch; > 0: the error it answers; -1: a block short
 int coop_calls = 0;
 cudaError_t __real_cudaLaunchCooperativeKernel(const void *, dim3, dim3, void **, size_t, cudaStream_t);
 cudaError_t __wrap_cudaLaunchCooperativeKernel(const void *f, dim3 g, dim3 b, void **a, size_t m, cudaStream_t s)
 {
     coop_calls++;
-    return coop_answer ? (cudaError_t)coop_answer : __real_cudaLaunchCooperativeKernel(f, g, b, a, m, s);
+    if (coop_answer < 0) g.x -= 1;
+    return coop_answer > 0 ? (cudaError_t)coop_answer : __real_cudaLaunchCooperativeKernel(f, g, b, a, m, s);
 }
 }
 """
@@ -108,4 +113,41 @@ def test_refused_launches_fall_back(refusing_library):
     # cudaErrorCooperativeLaunchTooLarge, cudaErrorNotSupported, cudaErrorNotPermitted
     r = subprocess.run([sys.executable, "-c", CHILD, ROOT, refusing_library, "720", "801", "800"], capture_output=True,
                        text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
+
+
+TIMEOUT_CHILD = r"""
+import ctypes as C, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+from pasc_inference_gb300 import capi
+capi.LIB_PATH = sys.argv[2]
+from pasc_inference_gb300 import PASC_PREC_MIXED, PascError, Problem
+answer = C.c_int.in_dll(capi.load(), "coop_answer")
+T, K = 20_000, 3
+rng = np.random.default_rng(1)
+x0 = rng.random(T * K)
+o = capi.spgqp_opts(maxit=3, m=10, eps=0.0)
+with Problem(T, K, 10.0, PASC_PREC_MIXED) as p:
+    p.set_data(rng.integers(0, K, T) + 0.5 * rng.standard_normal(T)); p.set_gamma(x0); p.set_theta(np.arange(K) + 0.1)
+    want = p.spgqp_solve(o).fx, p.get_gamma()
+    p.set_gamma(x0)
+    answer.value = -1
+    try:
+        p.spgqp_solve(o)
+    except PascError as e:
+        assert e.code == capi.PASC_ERR_TIMEOUT and "another block" in str(e), e
+    else:
+        raise AssertionError("no error")
+    answer.value = 0
+    p.set_gamma(x0)
+    assert p.spgqp_solve(o).fx == want[0]
+    assert np.array_equal(p.get_gamma(), want[1])
+print("ok")
+"""
+
+
+def test_wait_for_a_missing_block_is_reported(refusing_library):
+    r = subprocess.run([sys.executable, "-c", TIMEOUT_CHILD, ROOT, refusing_library], capture_output=True, text=True,
+                       timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
