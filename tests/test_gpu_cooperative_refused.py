@@ -18,6 +18,8 @@ import pytest
 
 from pasc_inference_gb300 import build as B
 
+pytestmark = pytest.mark.gpu
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 SHIM = r"""
