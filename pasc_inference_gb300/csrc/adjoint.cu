@@ -50,8 +50,10 @@ struct AdjointWork {
     long T = 0;
     double *gam = nullptr;           // N: FP64 gamma (the mixed path converts into it)
     double *gl = nullptr;            // N: dl/dgamma
-    double *lam = nullptr, *r = nullptr, *pb[2] = {nullptr, nullptr}, *q = nullptr;  // N each
-    float *r32 = nullptr, *pb32[2] = {nullptr, nullptr}, *q32 = nullptr, *d32 = nullptr;  // N each (mixed)
+    double *lam = nullptr, *r = nullptr;                      // N each
+    double *pb[2] = {nullptr, nullptr}, *q = nullptr;         // N each (FP64)
+    float *r32 = nullptr, *pb32[2] = {nullptr, nullptr}, *d32 = nullptr;  // N each (mixed)
+    float *q32 = nullptr;  // N (mixed; it and pb32[1] from the first solve over all timesteps on)
     cudaGraphExec_t chunk32 = nullptr;
     // mixed: the active timesteps, their number, and the words of the cooperative solve; r32, d32
     // and pb32[0] then hold n_active x K values
@@ -865,16 +867,16 @@ static int ensure_work(pasc_gb300_problem *p)
     w->grid = (int)std::max(1L, std::min((T + ADJ_NT - 1) / ADJ_NT, (long)p->sms * 4));
     auto dal = [&](void **ptr, size_t bytes) { return cudaMalloc(ptr, bytes > 0 ? bytes : 1) == cudaSuccess; };
     bool ok = dal((void **)&w->gl, sizeof(double) * N) && dal((void **)&w->lam, sizeof(double) * N) &&
-              dal((void **)&w->r, sizeof(double) * N) && dal((void **)&w->pb[0], sizeof(double) * N) &&
-              dal((void **)&w->pb[1], sizeof(double) * N) && dal((void **)&w->q, sizeof(double) * N) &&
-              dal((void **)&w->mask, sizeof(unsigned int) * T) && dal((void **)&w->clean, sizeof(double) * T) &&
+              dal((void **)&w->r, sizeof(double) * N) && dal((void **)&w->mask, sizeof(unsigned int) * T) && dal((void **)&w->clean, sizeof(double) * T) &&
               dal((void **)&w->dX, sizeof(double) * T) && dal((void **)&w->partials, sizeof(double) * 16 * w->grid) &&
               dal((void **)&w->out, sizeof(double) * 16) && dal((void **)&w->st, sizeof(AdjDevState)) &&
               dal((void **)&w->ticket, sizeof(unsigned int));
+    if (ok && p->precision != PASC_PREC_MIXED)
+        ok = dal((void **)&w->pb[0], sizeof(double) * N) && dal((void **)&w->pb[1], sizeof(double) * N) &&
+             dal((void **)&w->q, sizeof(double) * N);
     if (ok && p->precision == PASC_PREC_MIXED)
         ok = dal((void **)&w->gam, sizeof(double) * N) && dal((void **)&w->r32, sizeof(float) * N) &&
-             dal((void **)&w->pb32[0], sizeof(float) * N) && dal((void **)&w->pb32[1], sizeof(float) * N) &&
-             dal((void **)&w->q32, sizeof(float) * N) && dal((void **)&w->d32, sizeof(float) * N) &&
+             dal((void **)&w->pb32[0], sizeof(float) * N) && dal((void **)&w->d32, sizeof(float) * N) &&
              dal((void **)&w->list, sizeof(int) * T) && dal((void **)&w->counts, sizeof(int) * cg_list_counts(T)) &&
              dal((void **)&w->words, sizeof(unsigned long long) * cg_words(p->sms));
     if (ok) ok = cudaMallocHost((void **)&w->out_h, sizeof(double) * 16) == cudaSuccess &&
@@ -949,6 +951,11 @@ static int ensure_adj_graph32(pasc_gb300_problem *p)
     AdjointWork *w = p->adj;
     adj_drop_stale_graphs(p);
     if (w->chunk32) return PASC_OK;
+    for (float **v : {&w->pb32[1], &w->q32})
+        if (!*v && cudaMalloc((void **)v, sizeof(float) * p->N) != cudaSuccess) {
+            *v = nullptr;
+            return afail(PASC_ERR_ALLOC, "adjoint: device allocation failed");
+        }
     ACU(cudaStreamSynchronize(p->stream));
     cudaGraph_t g;
     ACU(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
