@@ -59,7 +59,7 @@ struct AdjointWork {
     // and pb32[0] then hold n_active x K values
     int *list = nullptr, *counts = nullptr, *n_h = nullptr;
     unsigned long long *words = nullptr;
-    unsigned int tag = 1;
+    WordTags tags;
     bool cg_fits = false, cg_refused = false;
     CgPlan cg{};
     int n_active = 0;
@@ -1028,7 +1028,6 @@ static int adj_refine(pasc_gb300_problem *p, AdjDevState *h, int *launches)
                 a.d = w->d32;
                 a.st = w->st;
                 a.slots = w->words;
-                a.tag = w->tag;
                 a.T = p->T;
                 a.n = w->n_active;
                 a.C = w->cg.C;
@@ -1036,6 +1035,8 @@ static int adj_refine(pasc_gb300_problem *p, AdjDevState *h, int *launches)
                 a.iterations = ADJ_CG_ITERATIONS;
                 a.resume = resume ? 1 : 0;
                 a.coeff = (float)p->coeffA;
+                if (w->tags.take(ADJ_CG_ITERATIONS, &a.tag))
+                    ACU(cudaMemsetAsync(w->words, 0, sizeof(unsigned long long) * cg_words(p->sms), s));
                 const cudaError_t e = launch_cg(p->K, w->cg, a, s);
                 if (cooperative_refused(e) && !resume) {
                     // the device does not take the launch (an SM partition, say): all timesteps, from
@@ -1048,7 +1049,6 @@ static int adj_refine(pasc_gb300_problem *p, AdjDevState *h, int *launches)
                     continue;
                 }
                 ACU(e);
-                w->tag += ADJ_CG_ITERATIONS;
                 *launches += 1;
             } else {
                 ACU(cudaGraphLaunch(w->chunk32, s));

@@ -757,12 +757,13 @@ static int fp64_fused_run(pasc_gb300_problem *p, bool first, long n, bool *refus
         a.kc = p->tp ? p->tp_ck64 : nullptr;
         a.st = p->st64;
         a.slots = p->res_slots;
-        a.tag = p->res_tag;
         a.T = p->T;
         a.C = p->f64_plan.C;
         a.trees = p->f64_plan.trees;
         a.first = begin ? 1 : 0;
         a.sweeps = (int)std::min(left, most);
+        if (p->res_tags.take((unsigned int)a.sweeps + 1, &a.tag))
+            CU(cudaMemsetAsync(p->res_slots, 0, fp64_words(p->sms) * sizeof *p->res_slots, s));
         const cudaError_t e = launch_fp64_iterations(p->K, p->f64_plan, a, s);
         if (cooperative_refused(e) && begin) {
             cudaGetLastError();
@@ -770,7 +771,6 @@ static int fp64_fused_run(pasc_gb300_problem *p, bool first, long n, bool *refus
             return PASC_OK;
         }
         if (e != cudaSuccess) return fail(PASC_ERR_CUDA, "fp64 iterations: %s", cudaGetErrorString(e));
-        p->res_tag += (unsigned int)a.sweeps + 1;
         left -= a.sweeps;
         begin = false;
         r.launches++;
@@ -1335,7 +1335,8 @@ static int resident_run(pasc_gb300_problem *p, bool init, long n)
         a.edge_hi = k_edge * W;
         a.init = init && launches == 0 ? 1 : 0;
         a.sweeps = (int)(left < RESIDENT_MAX_SWEEPS ? left : RESIDENT_MAX_SWEEPS);
-        a.tag = p->res_tag;
+        if (p->res_tags.take((unsigned int)a.sweeps, &a.tag))
+            CU(cudaMemsetAsync(p->res_slots, 0, resident_words(p->sms) * sizeof *p->res_slots, s));
         cudaError_t e = launch_resident(p->K, p->res_mode, p->res_plan, a, s);
         if (cooperative_refused(e) && launches == 0) {
             cudaGetLastError();
@@ -1344,7 +1345,6 @@ static int resident_run(pasc_gb300_problem *p, bool init, long n)
             return PASC_OK;
         }
         if (e != cudaSuccess) return fail(PASC_ERR_CUDA, "resident solve: %s", cudaGetErrorString(e));
-        p->res_tag += (unsigned int)a.sweeps;
         left -= a.sweeps;
         launches++;
         CU(cudaEventRecord(p->ev1, s));

@@ -5,6 +5,7 @@
 #include <float.h>
 
 #include "internal.h"
+#include "launch_rules.h"
 
 namespace pasc {
 struct AdjointWork;  // adjoint.cu
@@ -74,7 +75,7 @@ struct pasc_gb300_problem {
     // solves that run as one cooperative launch (kernels_resident.cu): used while the kernel is
     // left to the library (variant -1) and the state fits in shared memory
     unsigned long long *res_slots = nullptr;  // words of the cooperative launches (both precisions)
-    unsigned int res_tag = 1;     // tag of the next launch's first sweep
+    pasc::WordTags res_tags;      // of their sweeps
     int smem_optin = 0;
     int res_mode = -1;            // the form res_plan and the kernel attributes were made for
     bool res_fits = false, res_refused = false;

@@ -43,3 +43,33 @@ def test_fem_sum_index_range(tmp_path):
         if max(T1, T2 * K) <= 10**9:  # nothing ordinary is refused
             assert ok, (T1, T2, K)
     assert got == [1, 1, 1, 1, 0, 0, 0, 0, 1, 0, 0]
+
+
+TAGS = r"""
+int main()
+{
+    // adjoint solves (16384 tags each) and mixed launches of 1 to 4097: past 2^32 tags several times
+    const unsigned int steps[] = {16384u, 4097u * 1021u, 1u << 31};
+    for (unsigned int step : steps) {
+        WordTags t;
+        unsigned long long last = 0, cleared = 0, launches = 0;
+        for (unsigned long long given = 0; given < 3ull << 32; launches++) {
+            const unsigned int n = step > 65536 ? step : step - (unsigned int)(launches % 3);
+            unsigned int first = 0;
+            if (t.take(n, &first)) {
+                cleared++;
+                last = 0;
+            }
+            // above every tag since the buffer was cleared, never 0, no wrap inside the launch
+            if (first <= last || (unsigned long long)first + n - 1 > UINT_MAX) return 1;
+            last = (unsigned long long)first + n - 1;
+            given += n;
+        }
+        printf("%llu\n", cleared);
+    }
+}
+"""
+
+
+def test_word_tags_never_repeat(tmp_path):
+    assert [int(v) >= 2 for v in _run(tmp_path, TAGS)] == [True] * 3
