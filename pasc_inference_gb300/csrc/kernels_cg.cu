@@ -7,14 +7,20 @@
 // alone, in the shared memory of the blocks, and an iteration (r and p to q = P A p and p'q; then d,
 // r and r'r) moves nothing through HBM.  Block b owns C consecutive entries of the list, thread i
 // M of them; rows are padded to an odd stride.  A neighbour in time that is not active has p = 0.
-// The two sums of an iteration are FP64 (three FP32 terms up to a warp, f3.cuh) and travel as tagged
-// words (grid_words.cuh) together with r at the block's two ends, from which the neighbours bring their
-// copies of p forward themselves.  Warp 0 adds the blocks' sums and forms alpha and beta.  Measured at
-// T = 1e6, K = 3, 280 000 active timesteps: 26 us per iteration with one kernel per half iteration over all
-// timesteps, 6.9 here; 4.5 on eleven blocks, about 4 on one.  What bounds it: the two exchanges, 1.5 to 1.8 us each
-// between the two dies, and on few blocks warp 0's chain of FP64 operations (float-float sums and
-// quotients in every thread, with fewer bits, took 0.9 to 1.3 us less there, and up to 1.1 us more where many
-// entries share a block: T = 3e5, K = 8 7.1 against 5.9 ms an adjoint).
+// The two sums of an iteration are three FP32 terms (f3.cuh), closer than FP64 and without the chains of
+// the slow FP64 pipe; a block's sum is rounded to 48 bits once, when it is published.  They travel as
+// tagged words (grid_words.cuh) together with r at the block's two ends, from which the neighbours bring
+// their copies of p forward themselves.  Warp 0 adds the blocks' sums and forms alpha and beta; one block
+// needs no exchange, and every warp does it for itself.
+//
+// Measured, loss and gradient (ms): two kernels per iteration over all timesteps / float-float sums, added
+// and divided in every thread / here.  T = 1e6, K = 3, 643 iterations over 280 000 active timesteps 23.6 / 6.7 /
+// 6.2; T = 3e5, K = 8 39 / 7.1 / 5.4; T = 1e5, K = 2 3.1 / 1.48 / 1.15; T = 3e4, K = 3 6.4 / 3.5 / 2.5; T = 1e4, K = 2 2.3 /
+// 0.74 / 0.80; T = 5000, K = 3 3.7 / 1.07 / 1.36; T = 1000, K = 2 1.8 / 0.59 / 0.59.  What bounds it: the two
+// exchanges, 1.5 to 1.8 us each between the two dies, and on few entries the chain of the sums (13 steps of
+// a shuffle and 14 additions each).  How the blocks' polls fall between one another moves a solve on 2 to 32
+// blocks by up to a third from one GPU to another.  FP64 sums in place of the three terms: 0.9 to 1.3 us more
+// per iteration.
 //
 // The scalars follow adjoint.cu: alpha = r'r / p'q, beta the ratio of successive r'r, until r'r has
 // dropped by ADJ_INNER_TOL^2, maxit, or a breakdown (p'q <= 0).
@@ -29,7 +35,7 @@
 namespace pasc {
 
 constexpr int CG_NT = 512;
-constexpr int CG_WORDS = 4 + 2 * KMAX_FUSED;  // a block's words: two sums (FP64), r at its two ends
+constexpr int CG_WORDS = 4 + 2 * KMAX_FUSED;  // a block's words: two sums (high and low parts), r at its two ends
 
 // entry flags above the mask's bits
 constexpr unsigned int CG_LEFT = 1u << 8, CG_RIGHT = 1u << 9;    // the timestep has one before / after it
@@ -38,33 +44,32 @@ constexpr unsigned int CG_LACT = 1u << 10, CG_RACT = 1u << 11;  // which is the 
 template <int K>
 struct CgSmem {
     float hr[2][K], hp[2][K];  // r, p of the entries before and after the block
-    float red[CG_NT / 32][3];  // the warps' sums
-    // of the whole grid, from warp 0
+    float red[2][CG_NT / 32][3];  // the warps' sums (p'q, r'r)
+    float red2[CG_NT / 32][3];    // sums over 32 blocks each
+    // of several blocks, from warp 0
     float alpha, beta;
-    int status, it;
+    int status;
     int gave_up;               // a wait gave up
 };
 
-// sum over lanes 0 .. n - 1 (the others hold 0), in lane 0
-__device__ __forceinline__ double warp_sum_of(double v, int n)
+// a three-term sum as the nearest FP32 number and the rest
+__device__ __forceinline__ FF ff_of(F3 v)
 {
-    for (int m = n > 16 ? 16 : (n > 8 ? 8 : (n > 4 ? 4 : (n > 2 ? 2 : 1))); m >= 1; m >>= 1)
-        v += __shfl_xor_sync(0xffffffffu, v, m);
-    return v;
+    float e;
+    const float hi = f3_two_sum(v.a, v.b, e), r = e + v.c, h = hi + r;
+    return FF{h, r - (h - hi)};
 }
 
-// (float)(a / b).  A quotient of FP32 numbers and one correction from its FP64 remainder: off by 2^-46
-// before it is rounded to FP32.  (An FP64 division in its place: 0.2 to 0.4 us
-// more per iteration.)
-__device__ __forceinline__ float cg_quotient(double a, double b)
+// a / b rounded to FP32, inv = __frcp_rn(b.hi): a quotient of the high parts and one correction from its
+// remainder, off by 2^-44 before it is rounded
+__device__ __forceinline__ float ff_quotient(FF a, FF b, float inv)
 {
-    const float fa = (float)a, fb = (float)b;
-    if (!(fabsf(fa) > 0x1p-60f && fabsf(fa) < 0x1p60f && fabsf(fb) > 0x1p-60f && fabsf(fb) < 0x1p60f)) return (float)(a / b);
-    const float q = fa / fb;
-    return q + (float)fma(-(double)q, b, a) / fb;
+    const float q = __fmul_rn(a.hi, inv);
+    const float rem = __fadd_rn(__fadd_rn(fmaf(-q, b.hi, a.hi), a.lo), -__fmul_rn(q, b.lo));
+    return fmaf(rem, inv, q);
 }
 
-// A warp's share of a grid-wide sum: three FP32 terms within the warp (f3.cuh), FP64 beyond.
+// A warp's share of a grid-wide sum.
 __device__ __forceinline__ void cg_warp_sum(F3 v, float (*red)[3])
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -77,37 +82,69 @@ __device__ __forceinline__ void cg_warp_sum(F3 v, float (*red)[3])
     }
 }
 
-// Warp 0: the sum over the block's warps, published, and the sum over all blocks, in lane 0.
-// slots: the blocks' words (CG_WORDS apart), which: the sum's place among them.  ok turns false
-// where a wait gave up.
-__device__ __forceinline__ double cg_grid_sum(const float (*red)[3], unsigned long long *slots, int which,
-                                              unsigned int tag, bool &ok)
+// the sum over the block's warps (16 at most), in every lane of a warp: lanes 8 or 16 apart hold the same
+__device__ __forceinline__ F3 cg_block_sum(const float (*red)[3])
 {
-    constexpr int POLL = 5;  // words a lane has in flight
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, nb = gridDim.x;
-    const double own = warp_sum_of(lane < nw ? f3_value(F3{red[lane][0], red[lane][1], red[lane][2]}) : 0.0, nw);
-    if (nb == 1) return own;
-    if (lane == 0) word_store_double(slots + (size_t)blockIdx.x * CG_WORDS + 2 * which, own, tag);
-    double sum = 0.0;
-    for (int b0 = lane; b0 < nb; b0 += 32 * POLL) {
-        unsigned long long hi[POLL], lo[POLL];
+    const int nw = blockDim.x >> 5, w = threadIdx.x & (nw > 8 ? 15 : 7);
+    F3 v = w < nw ? F3{red[w][0], red[w][1], red[w][2]} : F3{0.f, 0.f, 0.f};
+    if (nw > 8) v = f3_add(v, f3_shfl_xor(v, 8));
+#pragma unroll
+    for (int m = 4; m >= 1; m >>= 1) v = f3_add(v, f3_shfl_xor(v, m));
+    return v;
+}
+
+// Several blocks: warp 0 publishes the block's sum, the first warps ask for the others' (one block per
+// lane, so that a word is read until it is there and no longer), and warp 0 returns the sum over all
+// blocks.  slots: the blocks' words (CG_WORDS apart), which: the sum's place among them.  A block's sum is
+// rounded to 48 bits when it is published, once.  gave_up is set where a wait gave up.
+__device__ __forceinline__ F3 cg_grid_sum(const float (*red)[3], float (*red2)[3], unsigned long long *slots, int which,
+                                          unsigned int tag, int &gave_up)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = gridDim.x, polling = (nb + 31) >> 5;
+    if (warp == 0) {
+        const FF p = ff_of(cg_block_sum(red));
+        if (lane == 0)
+            word_store2(slots + (size_t)blockIdx.x * CG_WORDS + 2 * which, word_of(p.hi, tag), word_of(p.lo, tag));
+    }
+    F3 sum{0.f, 0.f, 0.f};
+    if (tid < nb) {
+        const unsigned long long *w = slots + (size_t)tid * CG_WORDS + 2 * which;
+        unsigned long long hi = 0, lo = 0;
         bool have = false;
         for (unsigned int it = 0; it < WORD_WAIT_LIMIT && !have; it++) {
-            have = true;
-#pragma unroll
-            for (int q = 0; q < POLL; q++) {
-                const int b = b0 + 32 * q;
-                if (b < nb) word_load2(slots + (size_t)b * CG_WORDS + 2 * which, hi[q], lo[q]);
-                else hi[q] = lo[q] = word_of(0u, tag);
-            }
-#pragma unroll
-            for (int q = 0; q < POLL; q++) have &= word_valid(hi[q], tag) && word_valid(lo[q], tag);
+            word_load2(w, hi, lo);
+            have = word_valid(hi, tag) && word_valid(lo, tag);
         }
-        ok &= have;
-#pragma unroll
-        for (int q = 0; q < POLL; q++) sum += __hiloint2double((int)(unsigned int)hi[q], (int)(unsigned int)lo[q]);
+        if (!have) gave_up = 1;
+        sum = F3{word_float(hi), word_float(lo), 0.f};
     }
-    return warp_sum_of(sum, nb);
+    if (warp < polling) {
+        const int n = min(nb - 32 * warp, 32);  // lanes with a block
+        __syncwarp();
+        for (int m = n > 16 ? 16 : (n > 8 ? 8 : (n > 4 ? 4 : (n > 2 ? 2 : 1))); m >= 1; m >>= 1)
+            sum = f3_add(sum, f3_shfl_xor(sum, m));
+        if (polling > 1) {
+            if (lane == 0) {
+                red2[warp][0] = sum.a;
+                red2[warp][1] = sum.b;
+                red2[warp][2] = sum.c;
+            }
+            asm volatile("bar.sync 1, %0;" ::"r"(32 * polling) : "memory");
+            if (warp == 0) {
+                sum = lane < polling ? F3{red2[lane][0], red2[lane][1], red2[lane][2]} : F3{0.f, 0.f, 0.f};
+                for (int m = polling > 4 ? (polling > 8 ? 8 : 4) : 2; m >= 1; m >>= 1) sum = f3_add(sum, f3_shfl_xor(sum, m));
+            }
+        }
+    }
+    return sum;
+}
+
+// after an update of r (r'r = v; rr before it, inv_rr its reciprocal): beta, and whether the solve goes on
+__device__ __forceinline__ int cg_step(FF v, FF rr, float inv_rr, FF lim, bool last, float &beta)
+{
+    beta = ff_quotient(v, rr, inv_rr);
+    if (!isfinite(v.hi)) return ADJ_BREAKDOWN;
+    return (v.hi - lim.hi) + (v.lo - lim.lo) <= 0.f || last ? ADJ_INNER_DONE : ADJ_RUNNING;
 }
 
 template <int K>
@@ -148,8 +185,10 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
     float *r = rs + tid * S, *p = ps + tid * S, *q = qs + tid * S, *d = ds + tid * S;
     const unsigned short *fl = fs + tid * M;
     const float coeff = a.coeff;
-    double rr = a.st->rr;  // (thread 0)
-    const double stop = ADJ_INNER_TOL * ADJ_INNER_TOL * a.st->rr_in0;
+    const double rr_in = a.st->rr, stop = ADJ_INNER_TOL * ADJ_INNER_TOL * a.st->rr_in0;
+    // r'r (thread 0's counts; with one block all threads hold the same)
+    FF rr{(float)rr_in, (float)(rr_in - (double)(float)rr_in)};
+    const FF lim{(float)stop, (float)(stop - (double)(float)stop)};
     const int maxit = a.st->maxit;
     int it = a.st->it, status = ADJ_RUNNING;
     float beta = a.resume ? (float)a.st->beta : 0.f;
@@ -160,6 +199,7 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
     for (int s = 0; s < a.iterations; s++) {
         const unsigned int tag = a.tag + (unsigned int)s;
         unsigned long long *slots = a.slots + (size_t)(tag & 1u) * nb * CG_WORDS;
+        const float inv_rr = __frcp_rn(rr.hi);
         // p = r + beta p at the thread's entries and the ones beside them
         float pc[K], pl[K], pe[K];
         if (m > 0) {
@@ -211,23 +251,30 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
                 pq = f3_add(pq, part);
             }
         }
-        cg_warp_sum(pq, sm.red);
+        cg_warp_sum(pq, sm.red[0]);
         __syncthreads();
-        if (tid < 32) {
-            const double sum = cg_grid_sum(sm.red, slots, 0, tag, ok);
-            if (!__all_sync(0xffffffffu, ok)) sm.gave_up = 1;
+        float alpha;
+        if (nb == 1) {  // every warp for itself
+            const FF sum = ff_of(cg_block_sum(sm.red[0]));
+            if (!(sum.hi > 0.f) || !isfinite(sum.hi)) {
+                status = ADJ_BREAKDOWN;
+                break;
+            }
+            alpha = ff_quotient(rr, sum, __frcp_rn(sum.hi));
+        } else {
+            const FF sum = ff_of(cg_grid_sum(sm.red[0], sm.red2, slots, 0, tag, sm.gave_up));
             if (tid == 0) {
-                const bool fine = sum > 0.0 && isfinite(sum);
-                sm.alpha = fine ? cg_quotient(rr, sum) : 0.f;
+                const bool fine = sum.hi > 0.f && isfinite(sum.hi);
+                sm.alpha = fine ? ff_quotient(rr, sum, __frcp_rn(sum.hi)) : 0.f;
                 sm.status = fine ? ADJ_RUNNING : ADJ_BREAKDOWN;
             }
+            __syncthreads();
+            ok = sm.gave_up == 0;
+            if (!ok) break;
+            status = sm.status;
+            if (status != ADJ_RUNNING) break;
+            alpha = sm.alpha;
         }
-        __syncthreads();
-        ok = sm.gave_up == 0;
-        if (!ok) break;
-        status = sm.status;
-        if (status != ADJ_RUNNING) break;
-        const float alpha = sm.alpha;
         F3 rn{0.f, 0.f, 0.f};
 #pragma unroll 1
         for (int j = 0; j < m; j++) {
@@ -263,24 +310,23 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
                 sm.hr[e][k] = word_float(v);
             }
         }
-        cg_warp_sum(rn, sm.red);
+        cg_warp_sum(rn, sm.red[1]);
         __syncthreads();
-        if (tid < 32) {
-            const double sum = cg_grid_sum(sm.red, slots, 1, tag, ok);
-            if (!__all_sync(0xffffffffu, ok)) sm.gave_up = 1;
-            if (tid == 0) {
-                sm.beta = cg_quotient(sum, rr);
-                sm.it = it + 1;
-                sm.status = !isfinite(sum) ? ADJ_BREAKDOWN : (sum <= stop || it + 1 >= maxit ? ADJ_INNER_DONE : ADJ_RUNNING);
-            }
+        it++;
+        if (nb == 1) {
+            const FF sum = ff_of(cg_block_sum(sm.red[1]));
+            status = cg_step(sum, rr, inv_rr, lim, it >= maxit, beta);
             rr = sum;
+        } else {
+            const FF sum = ff_of(cg_grid_sum(sm.red[1], sm.red2, slots, 1, tag, sm.gave_up));
+            if (tid == 0) sm.status = cg_step(sum, rr, inv_rr, lim, it >= maxit, sm.beta);
+            rr = sum;
+            __syncthreads();
+            ok = sm.gave_up == 0;
+            if (!ok) break;
+            status = sm.status;
+            beta = sm.beta;
         }
-        __syncthreads();
-        ok = sm.gave_up == 0;
-        if (!ok) break;
-        status = sm.status;
-        beta = sm.beta;
-        it = sm.it;
         if (status != ADJ_RUNNING) break;
     }
     if (!ok) {
@@ -304,7 +350,7 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
         }
     }
     if (blockIdx.x == 0 && tid == 0) {
-        a.st->rr = rr;
+        a.st->rr = ff_value(rr);
         a.st->beta = beta;
         a.st->it = it;
         a.st->status = status;
@@ -405,8 +451,8 @@ static const void *cg_kernel_of(int K)
 
 size_t cg_words(int sms) { return (size_t)2 * sms * CG_WORDS; }
 
-// One block up to 512 entries, then 256 entries per block up to one block per SM; false where the
-// entries do not fit in shared memory.
+// One block up to 512 entries (K <= 4: 1024), then 256 entries per block up to one block per SM; false where
+// the entries do not fit in shared memory.
 bool cg_plan(int K, long n, int sms, CgPlan *p)
 {
     const void *fn = cg_kernel_of(K);
@@ -417,14 +463,15 @@ bool cg_plan(int K, long n, int sms, CgPlan *p)
         cudaGetLastError();
         return false;
     }
-    const long nb = n <= 512 ? 1 : std::min((long)sms, (n + 255) / 256);
+    const long nb = n <= (K <= 4 ? 1024 : 512) ? 1 : std::min((long)sms, (n + 255) / 256);
     const long C = (n + nb - 1) / nb, M = (C + CG_NT - 1) / CG_NT, rows = (C + M - 1) / M;
     const size_t smem = sizeof(float) * 4 * rows * ((M * K) | 1) + sizeof(short) * rows * M, room = optin - fa.sharedSizeBytes;
     if (smem > room) return false;
     p->blocks = (int)((n + C - 1) / C);
     p->C = (int)C;
     p->M = (int)M;
-    p->threads = (int)((rows + 31) / 32) * 32;
+    // (at least the warps that poll the blocks' words)
+    p->threads = (int)std::max((rows + 31) / 32, (long)(p->blocks + 31) / 32) * 32;
     p->smem = smem;
     // (the same limit for every handle: all a block can have)
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room) != cudaSuccess ||
