@@ -134,6 +134,12 @@ __global__ void __launch_bounds__(FEM_NT) fem_sum_field_kernel(const float *__re
     F3 s{0.f, 0.f, 0.f};
 #pragma unroll 8
     for (int i = lo[j]; i < hi; i++) s = f3_add(s, __ldg(g1 + (long)i * K + k));
+    if (scale == 1.0 && isfinite(s.a)) {  // gamma: the nearest FP32 number, off the FP64 pipe
+        float r;
+        const float h = f3_two_sum(s.a, s.b, r);
+        g2[e] = h + (r + s.c);
+        return;
+    }
     double sum = f3_value(s);
     if (!isfinite(s.a)) {  // beyond the FP32 range, or a value that is not finite
         sum = 0.0;
