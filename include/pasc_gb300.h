@@ -59,8 +59,9 @@ enum pasc_gb300_solve_status {
 
 /* Arithmetic of a handle. */
 enum pasc_gb300_precision {
-    PASC_PREC_FP64 = 0,     /* plain path: FP64 state, one kernel per reference operation,
-                               host-side step-length scalars (the reference's structure) */
+    PASC_PREC_FP64 = 0,     /* FP64 state and arithmetic in the reference's order; 1-D problems with
+                               K <= 8 iterate in one cooperative launch, others run one kernel
+                               per reference operation with host-side step-length scalars */
     PASC_PREC_MIXED = 1     /* fused path: FP32 gamma/gradient state, one HBM sweep per SPG
                                iteration, FP64 reductions and step lengths on the device */
 };
@@ -265,7 +266,7 @@ int pasc_gb300_get_fem(pasc_gb300_problem *p, double *fem_reduce, int *fem_type,
  * indices), each list sorted ascending, no duplicates, no self-loops, symmetric (checked;
  * PASC_ERR_ARG otherwise).  Image data (test_image): T = 1, R = width*height, the grid graph.
  * Not with FEM reduction, theta in the penalty, multichannel data or the adjoint
- * (PASC_ERR_NOTSUPP).  The mixed path runs two kernels per SPG iteration. */
+ * (PASC_ERR_NOTSUPP).  The mixed path runs two kernels per SPG iteration (an image: one). */
 int pasc_gb300_create_graph(pasc_gb300_problem **out, long T, long R, int K, int precision, double epssqr,
                             int device, const int *nbr_ptr, const int *nbr_idx);
 /* T = timesteps, R = nodes (1 and 0 edges for a 1-D problem) */

@@ -112,9 +112,9 @@ __global__ void fem_prolongate_kernel(const TIn *g2, TOut *g1, long T1, long T2,
 // where the first value lies far from all others that is n digits' worth of cancellation, and
 // infinities give inf - inf.  Where the sum is below 2^-8 of S2 (c some 16 standard deviations off) or not a
 // number it is therefore taken term by term; elsewhere at most 11 of FP64's 53 bits are lost of a sum that
-// is stored in 24.  (One thread per coarse entry,
-// summing in FP64 with a stride of K: 95 us for both reductions at T = 2e6, K = 3, T2 = T/10; here
-// 24 and 12, and the copy back 15.)
+// is stored in 24.
+// Both reductions at T = 2e6, K = 3, one thread per coarse entry summing in FP64 with a stride of K / float-float
+// sums / here: T2 = T/10 95 / 42 / 41 us, T2 = T/2 180 / 89 / 75.  The copy back: 15.
 constexpr int FEM_NT = (int)FEM_SUM_THREADS;
 
 __global__ void __launch_bounds__(FEM_NT) fem_bounds_kernel(int *lo, long T2, double diff)
