@@ -796,8 +796,6 @@ static int fp64_fused_run(pasc_gb300_problem *p, bool first, long n, bool *refus
     r.fx_old = h->fx_old;
     r.dd = h->dd_done;
     r.dAd = h->dAd_done;
-    p->fx_last = r.fx;
-    p->have_fx = true;
     return PASC_OK;
 }
 
@@ -908,6 +906,8 @@ static int fp64_iterate(pasc_gb300_problem *p, long n)
             CHK(fp64_fused_run(p, false, n, &refused));
         }
         if (r.status == PASC_SPG_RUNNING && r.it >= o->maxit) r.status = PASC_SPG_MAXIT;
+        p->fx_last = r.fx;
+        p->have_fx = true;
         return PASC_OK;
     }
     // SPGQPSolverC (spgqpsolver_coeff.h:611-835): d'Ad, the BB step and the A-condition without

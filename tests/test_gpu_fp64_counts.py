@@ -6,7 +6,7 @@ for it."""
 import numpy as np
 import pytest
 
-from pasc_inference_gb300 import PASC_PREC_FP64, Problem, capi
+from pasc_inference_gb300 import PASC_PREC_FP64, PascError, Problem, capi
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +52,21 @@ def test_a_vanished_direction_is_reported_by_the_call_that_asks_for_it(gpulib, K
             assert (st.it, st.hessmult, st.status) == (whole.it, whole.it + 2, capi.PASC_SPG_DAD_ZERO)
         assert st.fx == whole.fx and st.gP == whole.gP
         np.testing.assert_array_equal(p.get_gamma(), g)
+
+
+@pytest.mark.parametrize("K", [3, 9])
+def test_get_fx_belongs_to_iterate(gpulib, K):
+    """The objective is handed out after an iterate call, not after a start alone."""
+    p, x0 = _problem(300, K)
+    with p:
+        p.spgqp_start(capi.spgqp_opts(maxit=10, m=10, eps=0.0))
+        with pytest.raises(PascError) as e:
+            p.get_fx()
+        assert e.value.code == capi.PASC_ERR_STATE
+        st = p.spgqp_iterate(0)
+        assert p.get_fx() == st.fx
+        st = p.spgqp_iterate(3)
+        assert p.get_fx() == st.fx
+        p.set_gamma(x0)
+        st = p.spgqp_solve(capi.spgqp_opts(maxit=5, m=10, eps=0.0))
+        assert p.get_fx() == st.fx
