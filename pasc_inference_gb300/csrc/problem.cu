@@ -1419,7 +1419,12 @@ static int mixed_iterate(pasc_gb300_problem *p, long n, int poll)
     const long room = p->run.o.maxit - p->run.it;
     if (n > room) n = room;
     if (p->res_used) {
-        if (n > 0) CHK(resident_run(p, false, n));
+        if (n > 0) {
+            CHK(resident_run(p, false, n));
+        } else {
+            p->run.last_iterate_ms = 0.f;
+            p->run.last_iterate_launches = 0;
+        }
         if (!p->res_used) return fail(PASC_ERR_STATE, "spgqp_iterate: the device no longer takes the cooperative launch this solve began with");
         if (p->run.status == PASC_SPG_RUNNING && p->run.it >= p->run.o.maxit) p->run.status = PASC_SPG_MAXIT;
         return PASC_OK;

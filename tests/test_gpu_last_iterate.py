@@ -39,3 +39,5 @@ def test_solve_in_one_launch(gpulib):
         st = p.spgqp_iterate(2)
         ms, n = p.spgqp_last_iterate()
         assert st.it == 2 and n == 1 and 0.0 < ms * 1e-3 < st.time_s
+        p.spgqp_iterate(0)  # nothing of the call before is left over
+        assert p.spgqp_last_iterate() == (0.0, 0)
