@@ -61,9 +61,11 @@ __device__ __forceinline__ FF ff_of(F3 v)
 }
 
 // a / b rounded to FP32, inv = __frcp_rn(b.hi): a quotient of the high parts and one correction from its
-// remainder, off by 2^-44 before it is rounded
+// remainder, off by 2^-44 before it is rounded (b far from 1: FP64, so that inv neither overflows nor is
+// subnormal)
 __device__ __forceinline__ float ff_quotient(FF a, FF b, float inv)
 {
+    if (!(b.hi > 0x1p-100f && b.hi < 0x1p100f)) return (float)(ff_value(a) / ff_value(b));
     const float q = __fmul_rn(a.hi, inv);
     const float rem = __fadd_rn(__fadd_rn(fmaf(-q, b.hi, a.hi), a.lo), -__fmul_rn(q, b.lo));
     return fmaf(rem, inv, q);
