@@ -15,12 +15,12 @@
 //
 // Measured, loss and gradient (ms): two kernels per iteration over all timesteps / float-float sums, added
 // and divided in every thread / here.  T = 1e6, K = 3, 643 iterations over 280 000 active timesteps 23.6 / 6.7 /
-// 6.2; T = 3e5, K = 8 39 / 7.1 / 5.4; T = 1e5, K = 2 3.1 / 1.48 / 1.15; T = 3e4, K = 3 6.4 / 3.5 / 2.5; T = 1e4, K = 2 2.3 /
-// 0.74 / 0.80; T = 5000, K = 3 3.7 / 1.07 / 1.36; T = 1000, K = 2 1.8 / 0.59 / 0.59.  What bounds it: the two
+// 6.1; T = 3e5, K = 8 39 / 7.1 / 5.2; T = 1e5, K = 2 3.1 / 1.48 / 1.08; T = 3e4, K = 3 6.4 / 3.5 / 2.35; T = 1e4, K = 2 2.3 /
+// 0.74 / 0.77; T = 5000, K = 3 3.7 / 1.07 / 1.29; T = 1000, K = 2 1.8 / 0.59 / 0.59.  What bounds it: the two
 // exchanges, 1.5 to 1.8 us each between the two dies, and on few entries the chain of the sums (13 steps of
 // a shuffle and 14 additions each).  How the blocks' polls fall between one another moves a solve on 2 to 32
 // blocks by up to a third from one GPU to another.  FP64 sums in place of the three terms: 0.9 to 1.3 us more
-// per iteration.
+// per iteration.  The neighbours' r awaited before a block publishes its sum: 0.2 to 0.7 us more.
 //
 // The scalars follow adjoint.cu: alpha = r'r / p'q, beta the ratio of successive r'r, until r'r has
 // dropped by ADJ_INNER_TOL^2, maxit, or a breakdown (p'q <= 0).
@@ -297,21 +297,6 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
             }
             rn = f3_add(rn, part);
         }
-        // (the neighbours' r at this block's ends are awaited with the sum)
-        if (nb > 1 && tid >= nt - 2 * K) {
-            const int e = (tid - (nt - 2 * K)) / K, k = tid - (nt - 2 * K) - e * K, ob = (int)blockIdx.x + (e ? 1 : -1);
-            if (ob >= 0 && ob < nb) {
-                const unsigned long long *w = slots + (size_t)ob * CG_WORDS + 4 + (e ? 0 : K) + k;
-                unsigned long long v = 0;
-                bool have = false;
-                for (unsigned int n = 0; n < WORD_WAIT_LIMIT && !have; n++) {
-                    v = word_load(w);
-                    have = word_valid(v, tag);
-                }
-                if (!have) sm.gave_up = 1;
-                sm.hr[e][k] = word_float(v);
-            }
-        }
         cg_warp_sum(rn, sm.red[1]);
         __syncthreads();
         it++;
@@ -320,6 +305,22 @@ __global__ void __launch_bounds__(CG_NT, 1) cg_resident_kernel(const __grid_cons
             status = cg_step(sum, rr, inv_rr, lim, it >= maxit, beta);
             rr = sum;
         } else {
+            // the neighbours' r at this block's ends, awaited beside the sum (by the last warp: the
+            // block's own share is published first)
+            if (tid >= nt - 2 * K) {
+                const int e = (tid - (nt - 2 * K)) / K, k = tid - (nt - 2 * K) - e * K, ob = (int)blockIdx.x + (e ? 1 : -1);
+                if (ob >= 0 && ob < nb) {
+                    const unsigned long long *w = slots + (size_t)ob * CG_WORDS + 4 + (e ? 0 : K) + k;
+                    unsigned long long v = 0;
+                    bool have = false;
+                    for (unsigned int n = 0; n < WORD_WAIT_LIMIT && !have; n++) {
+                        v = word_load(w);
+                        have = word_valid(v, tag);
+                    }
+                    if (!have) sm.gave_up = 1;
+                    sm.hr[e][k] = word_float(v);
+                }
+            }
             const FF sum = ff_of(cg_grid_sum(sm.red[1], sm.red2, slots, 1, tag, sm.gave_up));
             if (tid == 0) sm.status = cg_step(sum, rr, inv_rr, lim, it >= maxit, sm.beta);
             rr = sum;
